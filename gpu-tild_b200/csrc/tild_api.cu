@@ -111,11 +111,12 @@ void free_all(tild_ctx* c) {
   for (Bucket& b : c->buckets)
     if (b.planned) {
       cufftDestroy(b.fwd_packed ? b.c2c_fwd : b.r2c);
-      cufftDestroy(b.packed ? b.c2c : b.c2r);
+      if (!b.own) cufftDestroy(b.packed ? b.c2c : b.c2r);
     }
   for (auto& ge : c->graphs) cudaGraphExecDestroy(ge.exec);
   c->graphs.clear();
   tild_sort_free(c);
+  tild_fft_free(c);
   for (cudaStream_t a : c->aux) cudaStreamDestroy(a);
   for (cudaEvent_t e : c->ev_join) cudaEventDestroy(e);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
@@ -227,7 +228,7 @@ int tild_assign_lanes(tild_ctx* c, int lanes) {
       b.lane = best;
       load[best] += work(bi);
     }
-    if (!b.planned) continue;
+    if (!b.planned || b.own) continue;  // own passes: the plan serves the observables, on the main stream
     cudaStream_t bs = b.lane >= 0 ? c->aux[b.lane] : c->stream;
     if (tild_check_fft(c, cufftSetStream(b.fwd_packed ? b.c2c_fwd : b.r2c, bs), "plan stream") ||
         tild_check_fft(c, cufftSetStream(b.packed ? b.c2c : b.c2r, bs), "plan stream"))
@@ -450,14 +451,30 @@ int engine_create(const tild_config* cfgs, int nsys, int device, tild_ctx* c, co
     // boundary (they are read as complex pairs); the pair spectra follow one another in rhok
     b.fwd_packed = b.packed && b.grid0 % 2 == 0;
     long long pairs = 0;
+    // A plain batch keeps the library transforms, whose results its members' long runs then reproduce
+    // bit for bit: with the own passes the forces differ by 2e-7 to 4e-7 (relative, as much as either is
+    // from 64 bits), which moved an ensemble's densities by 2e-5 to 4e-5 within 128 steps (296 against
+    // 471 us a step for 40 systems of 24^3 to 48^3).
+    b.own = nsys == 1 || capacity;
+    for (int s : b.systems) b.own = b.own && tild_fft_supports(b.nx, c->D, c->sys[s].T, c->sys[s].C);
     for (int s : b.systems) {
       const SysHost& h = c->sys[s];
+      if (b.own) {  // pair spectra and pair fields follow one another, an odd channel as a pair of its own
+        c->h_sys[s].inv_packed = 0;
+        c->h_sys[s].fwd_packed = b.fwd_packed ? 1 : 0;
+        c->h_sys[s].zk0 = b.spec0 + pairs * h.g.M;
+        c->h_sys[s].gkp0 = b.spec0 * c->D + pairs * c->D * h.g.M;
+        c->h_sys[s].rkp0 = c->h_sys[s].zk0;
+        pairs += (h.T + h.C + 1) / 2;
+        continue;
+      }
       c->h_sys[s].inv_packed = b.packed ? 1 : 0;
       c->h_sys[s].gkp0 = b.packed ? b.spec0 * c->D + pairs * c->D * h.g.M : 0;
       c->h_sys[s].fwd_packed = b.fwd_packed ? 1 : 0;
       c->h_sys[s].rkp0 = b.fwd_packed ? b.spec0 + pairs * h.g.M : 0;
       pairs += (h.T + h.C) / 2;
     }
+    if (b.own) spec = std::max(spec, b.spec0 + pairs * ((long long)b.nx[0] * b.nx[1] * b.nx[2]));
   }
   c->grid_total = grid;
   c->spec_total = spec;
@@ -505,7 +522,7 @@ int engine_create(const tild_config* cfgs, int nsys, int device, tild_ctx* c, co
   rc = rc ? rc : dalloc(c, &c->rhok, (size_t)spec, "density spectra");
   rc = rc ? rc : dalloc(c, &c->gk, (size_t)spec * c->D, "force spectra");
   bool any_c2r = false;  // planar force fields are only needed by buckets whose inverse is C2R
-  for (const Bucket& b : c->buckets) any_c2r = any_c2r || !b.packed;
+  for (const Bucket& b : c->buckets) any_c2r = any_c2r || (!b.packed && !b.own);
   rc = rc ? rc : dalloc(c, &c->gfield, any_c2r ? (size_t)grid * c->D : 1, "force fields");
   rc = rc ? rc : dalloc(c, &c->g4, (size_t)c->g4_total, "interleaved force fields");
   rc = rc ? rc : dalloc(c, &c->utab, (size_t)utab, "multiplier tables");
@@ -557,6 +574,11 @@ int engine_create(const tild_config* cfgs, int nsys, int device, tild_ctx* c, co
         ? cufftPlanMany(&b.c2c_fwd, c->D, n, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C, b.channels / 2)
         : cufftPlanMany(&b.r2c, c->D, n, nullptr, 1, 0, nullptr, 1, 0, CUFFT_R2C, b.channels);
     if (tild_check_fft(c, pf, b.fwd_packed ? "plan C2C forward" : "plan R2C")) return TILD_ERR_CUDA;
+    if (b.own) {
+      b.planned = true;
+      if (tild_check_fft(c, cufftSetStream(b.fwd_packed ? b.c2c_fwd : b.r2c, c->stream), "plan stream")) return TILD_ERR_CUDA;
+      continue;
+    }
     const cufftResult pi = b.packed
         ? cufftPlanMany(&b.c2c, c->D, n, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2C, b.channels / 2 * c->D)
         : cufftPlanMany(&b.c2r, c->D, n, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2R, b.channels * c->D);
@@ -567,6 +589,15 @@ int engine_create(const tild_config* cfgs, int nsys, int device, tild_ctx* c, co
     b.planned = true;
   }
   if (tild_assign_lanes(c, (int)c->aux.size())) return TILD_ERR_CUDA;
+  // several shapes on the library transforms: each shape's grid stages in sequence on its stream, so that
+  // small transforms overlap other shapes' passes (40 systems of 25 shapes: 411 against 486 us a step
+  // stage by stage; 8 systems of 8 shapes: 107 against 119).  Own passes take all shapes at once.
+  if (c->buckets.size() > 1) {
+    c->fft_pipeline = 1;
+    for (const Bucket& b : c->buckets)
+      if (b.own) c->fft_pipeline = 0;
+  }
+  rc = tild_fft_setup(c);
   for (int s = 0; s < nsys && !rc; s++) rc = tild_build_tables(c, s);
   if (rc) return rc;
   if (c->sort_interval > 0) {
@@ -741,7 +772,9 @@ int run_steps(tild_ctx* c, int n) {
       else if (n >= kMinGraphSteps) L = std::min(n, len);
     }
     if (L == 0) {
+      c->write_rho = n == 1;  // only the last step's densities can be read
       int rc = tild_run_forces(c, true, nullptr, -1);
+      c->write_rho = true;
       if (rc) return rc;
       n -= 1;
       continue;
@@ -778,7 +811,11 @@ int run_steps(tild_ctx* c, int n) {
     if (tild_check(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed), "begin capture"))
       return TILD_ERR_CUDA;
     int rc = TILD_OK;
-    for (int k = 0; k < L && !rc; k++) rc = tild_run_forces(c, true, nullptr, -1);
+    for (int k = 0; k < L && !rc; k++) {
+      c->write_rho = k == L - 1;
+      rc = tild_run_forces(c, true, nullptr, -1);
+    }
+    c->write_rho = true;
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
     if (rc) {

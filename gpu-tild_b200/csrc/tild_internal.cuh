@@ -66,6 +66,12 @@ struct SysDev {
   int fwd_packed;                  // 1: densities of channels (2c, 2c+1) are stored as one complex field
                                    //    (real, imaginary) and take one forward C2C
   long long rkp0;                  // with fwd_packed: this system's first pair spectrum in rhok (complex elements)
+  short fft_r1[3], fft_r2[3];      // with own grid passes: radices of each axis (tild_fft.cu)
+  int fft_tw[3], fft_twr;          //    the axis's unit roots in fft_twid, and x's by rows after them
+  int ztile;                       //    z pass: 0 multiplies style by style, 1 and 2 from ztab (2: beside the exchange)
+  short zramp[10];                 //    style whose ramp scales a pair of types (-1: none)
+  long long zt0;                   //    first multiplier in ztab
+  long long zk0;                   //    first pair spectrum in rhok (complex elements)
   long long g4_0, Mb;              // channel 0 in g4 and the per-channel stride there (>= M)
   long long utab0, ctab0, kd0;     // offsets in utab, ctab, kd
   long long step;                  // completed steps (advanced on the device)
@@ -119,6 +125,10 @@ struct Bucket {     // systems sharing one grid shape: one batched R2C plan and 
   bool fwd_packed = false;               // the forward transforms pair channels too (out of place C2C)
   cufftHandle r2c = 0, c2r = 0, c2c = 0, c2c_fwd = 0;
   bool planned = false;
+  // own grid passes (tild_fft.cu): the forward cuFFT plan serves the observables' spectra only
+  bool own = false;
+  bool spectra = false;                  // rhok holds the library spectra of the last force evaluation
+  int fft_blk0[5] = {0}, fft_nblk[5] = {0};
   int cta_spec0 = 0, n_cta_spec = 0;     // the shape's range of spectrum blocks (k-space multiply)
   int cta_grid0 = 0, n_cta_grid = 0;     // and of grid blocks (interleave)
   int cta_bead0 = 0, n_cta_bead = 0;     // and of particle blocks (spread, gather)
@@ -143,6 +153,17 @@ struct tild_ctx {
   int spread_ahead = 1;                  // integrating gathers spread x_{n+1} for the next step (order <= 1 default)
   bool rho_ahead = false;                // rho_fx already holds the densities of the current positions
   long long g4_total = 0;
+  struct FftPass {
+    int2* blocks = nullptr;              // {system, block of the system} per CTA
+    int n = 0;
+    size_t smem = 0;
+  };
+  FftPass fft_pass[5];                   // x, y forward, z with the multiply, y, x inverse
+  float2* fft_twid = nullptr;
+  float* ztab = nullptr;                 // multipliers in the z pass's order
+  bool fft_wide = false;                 // 16 columns per CTA in the y inverse pass
+  int fft_points = 1024;                 // points per field of an x pass's CTA
+  bool write_rho = true;                 // the next force evaluation stores the float densities
   int D = 3, P = 1;
   int nsys = 1;
   std::vector<SysHost> sys;
@@ -434,6 +455,12 @@ int tild_run_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys);   //
 int tild_finish_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys, bool interleaved, bool gathered);
 int tild_density_planar(tild_ctx* c, int s, float* dst, cudaStream_t st);                 // tild_step.cu
 const float2* tild_half_spectra(tild_ctx* c, int s);                                     // tild_step.cu
+bool tild_fft_supports(const int* nx, int D, int T, int C);
+int tild_fft_tables(tild_ctx* c, int s);                               // tild_fft.cu
+int tild_fft_setup(tild_ctx* c);
+void tild_fft_free(tild_ctx* c);
+int tild_fft_run(tild_ctx* c, const Bucket* b, bool integrate, bool active, cudaStream_t st);
+int tild_fieldphase_nodes(tild_ctx* c, const FieldK& fk);
 int tild_obs_compute(tild_ctx* c, int s, tild_obs* o); // tild_obs.cu
 int tild_sk_acc_run(tild_ctx* c, int s, int slot, int type);
 int tild_table_scratch(tild_ctx* c);

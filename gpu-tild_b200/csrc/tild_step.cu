@@ -355,6 +355,35 @@ __global__ void k_fix_to_pairs(unsigned long long* __restrict__ fx, float2* __re
   a[M] = 0ull;
 }
 
+// Both conversions over grid blocks [blk_off, ..) of any shapes in one launch: a CTA takes 256 nodes of
+// one system and all its channels (an ensemble of 25 grid shapes converted shape by shape spent
+// 100 us on 25 launches of 4 us).
+__global__ void __launch_bounds__(256) k_fix_nodes(unsigned long long* __restrict__ fx_all, float* __restrict__ rho_all,
+                                                   const int* __restrict__ cta_sys, const int* __restrict__ blk0,
+                                                   const SysDev* __restrict__ sysd, int blk_off) {
+  const int blk = blockIdx.x + blk_off, s = cta_sys[blk];
+  const SysDev& sd = sysd[s];
+  const long long M = sd.g.M, m = (long long)(blk - blk0[s]) * blockDim.x + threadIdx.x;
+  if (m >= M) return;
+  const int nch = sd.T + sd.C;
+  const bool paired = sd.fwd_packed;
+  unsigned long long* fx = fx_all + sd.grid0 + m;
+  float* rho = rho_all + sd.grid0;
+  for (int c = 0; c < nch; c += 2) {
+    const bool two = c + 1 < nch;
+    const long long va = (long long)fx[c * M], vb = two ? (long long)fx[(c + 1) * M] : 0;
+    fx[c * M] = 0ull;
+    if (two) fx[(c + 1) * M] = 0ull;
+    const float a = (float)((double)va * kInvFix), b = (float)((double)vb * kInvFix);
+    if (paired) {
+      reinterpret_cast<float2*>(rho + c * M)[m] = make_float2(a, b);
+    } else {
+      rho[c * M + m] = a;
+      if (two) rho[(c + 1) * M + m] = b;
+    }
+  }
+}
+
 // paired density spectra -> per-channel half spectra (the R2C layout, for the observables and S(k)):
 // one thread per half-spectrum point, every pair of the system
 __global__ void k_unpack_half(const float2* __restrict__ z, float2* __restrict__ half, int npairs, Geom g, int D) {
@@ -1391,6 +1420,7 @@ int tild_run_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys) {
     int rs = tild_sort_beads(c);
     if (rs) return rs;
   }
+  for (Bucket& b : c->buckets) b.spectra = !b.own;  // own passes keep no spectra
   const std::vector<char> on = integrate ? tild_buckets_on(c) : std::vector<char>(c->buckets.size(), 1);
   if (c->fft_pipeline >= 2 && c->lanes > 0 && c->fields.empty()) {
     // each grid shape runs its whole step in order on its stream: spread, conversion, R2C,
@@ -1408,8 +1438,12 @@ int tild_run_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys) {
         else dispatch_p_spread<2>(c, r);
         c->launches++;
       }
-      launch_fix(c, b, bs);
-      if (on[bi]) {
+      if (b.own) {
+        if (tild_fft_run(c, &b, integrate, on[bi], bs)) return TILD_ERR_CUDA;
+      } else {
+        launch_fix(c, b, bs);
+      }
+      if (on[bi] && !b.own) {
         if (exec_forward(c, b)) return TILD_ERR_CUDA;
         if (c->D == 3) launch_kmul<3>(c, integrate, bs, b.cta_spec0, b.n_cta_spec);
         else launch_kmul<2>(c, integrate, bs, b.cta_spec0, b.n_cta_spec);
@@ -1442,6 +1476,10 @@ int tild_run_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys) {
     for (size_t bi = 0; bi < c->buckets.size(); bi++) {
       const Bucket& b = c->buckets[bi];
       cudaStream_t bs = b.lane >= 0 ? c->aux[b.lane] : c->stream;
+      if (b.own) {
+        if (tild_fft_run(c, &b, integrate, on[bi], bs)) return TILD_ERR_CUDA;
+        continue;
+      }
       launch_fix(c, b, bs);
       if (!on[bi]) continue;
       if (exec_forward(c, b)) return TILD_ERR_CUDA;
@@ -1459,13 +1497,25 @@ int tild_run_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys) {
     if (tild_check(c, cudaGetLastError(), "shape pipeline")) return TILD_ERR_CUDA;
     return tild_finish_forces(c, integrate, f_bead, f_sys, c->fields.empty(), false);
   }
+  // stage by stage: the own passes of every shape that takes them, then the other shapes
+  if (tild_fft_run(c, nullptr, integrate, true, c->stream)) return TILD_ERR_CUDA;
+  bool any_lib = false;
+  for (const Bucket& b : c->buckets) any_lib = any_lib || !b.own;
+  if (!any_lib) return tild_finish_forces(c, integrate, f_bead, f_sys, true, false);
+  // runs of neighbouring shapes that take the library, in one launch each
+  struct Range { int g0, ng, s0, ns; };
+  std::vector<Range> runs;
+  bool open = false;
+  for (const Bucket& b : c->buckets) {
+    if (b.own) { open = false; continue; }
+    if (!open) runs.push_back({b.cta_grid0, 0, b.cta_spec0, 0});
+    open = true;
+    runs.back().ng += b.n_cta_grid;
+    runs.back().ns += b.n_cta_spec;
+  }
   tild_mark(c, STAGE_ZERO);
-  bool any_fwd_packed = false;
-  for (const Bucket& b : c->buckets) any_fwd_packed = any_fwd_packed || b.fwd_packed;
-  if (any_fwd_packed) {  // paired shapes convert into their own layout
-    for (const Bucket& b : c->buckets) launch_fix(c, b, c->stream);
-  } else {
-    k_fix_to_float<<<nblk(c->grid_total, 256), 256, 0, c->stream>>>(c->rho_fx, c->rho, c->grid_total);
+  for (const Range& r : runs) {
+    k_fix_nodes<<<r.ng, 256, 0, c->stream>>>(c->rho_fx, c->rho, c->cta_grid, c->cta_grid + c->n_cta_grid, c->d_sys, r.g0);
     c->launches++;
   }
   if (tild_check(c, cudaGetLastError(), "spread")) return TILD_ERR_CUDA;
@@ -1473,20 +1523,21 @@ int tild_run_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys) {
   if (fork(c)) return TILD_ERR_CUDA;
   for (size_t bi = 0; bi < c->buckets.size(); bi++) {
     const Bucket& b = c->buckets[bi];
-    if (on[bi] && exec_forward(c, b)) return TILD_ERR_CUDA;
+    if (on[bi] && !b.own && exec_forward(c, b)) return TILD_ERR_CUDA;
   }
   if (join(c)) return TILD_ERR_CUDA;
   tild_mark(c, STAGE_KMUL);
-  if (c->D == 3) launch_kmul<3>(c, integrate);
-  else launch_kmul<2>(c, integrate);
-  c->launches++;
+  for (const Range& r : runs) {
+    if (c->D == 3) launch_kmul<3>(c, integrate, c->stream, r.s0, r.ns);
+    else launch_kmul<2>(c, integrate, c->stream, r.s0, r.ns);
+    c->launches++;
+  }
   if (tild_check(c, cudaGetLastError(), "kmul")) return TILD_ERR_CUDA;
   tild_mark(c, STAGE_C2R);
   if (fork(c)) return TILD_ERR_CUDA;
   for (size_t bi = 0; bi < c->buckets.size(); bi++) {
     const Bucket& b = c->buckets[bi];
-    if (on[bi] && exec_inverse(c, b))
-      return TILD_ERR_CUDA;
+    if (on[bi] && !b.own && exec_inverse(c, b)) return TILD_ERR_CUDA;
   }
   if (join(c)) return TILD_ERR_CUDA;
   return tild_finish_forces(c, integrate, f_bead, f_sys, false, false);
@@ -1498,15 +1549,27 @@ int tild_finish_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys, bo
   if (!c->fields.empty()) tild_mark(c, STAGE_FIELD);
   for (const FieldK& fk : c->fields) {
     const SysHost& h = c->sys[fk.sys];
+    if (c->buckets[h.bucket].own) continue;  // added to the nodes below
     k_fieldphase_apply<<<nblk(h.g.M, 256), 256, 0, c->stream>>>(c->gfield + h.grid0 * c->D, c->rho + h.grid0,
                                                                  c->frfield + fk.fr0, fk.a, fk.b, c->D, h.g.M);
     c->launches++;
   }
   if (!interleaved) {
     tild_mark(c, STAGE_INTERLEAVE);
-    launch_interleave(c, c->stream, 0, c->n_cta_grid);
-    c->launches++;
+    for (size_t k = 0; k < c->buckets.size();) {  // neighbouring shapes that take the library in one launch
+      const int off = c->buckets[k].cta_grid0;
+      int n = 0;
+      for (; k < c->buckets.size() && !c->buckets[k].own; k++) n += c->buckets[k].n_cta_grid;
+      if (n) {
+        launch_interleave(c, c->stream, off, n);
+        c->launches++;
+      }
+      while (k < c->buckets.size() && c->buckets[k].own) k++;
+    }
   }
+  if (!c->fields.empty()) tild_mark(c, STAGE_FIELD);
+  for (const FieldK& fk : c->fields)
+    if (c->buckets[c->sys[fk.sys].bucket].own && tild_fieldphase_nodes(c, fk)) return TILD_ERR_CUDA;
   if (!gathered) {
     tild_mark(c, STAGE_GATHER);
     if (c->D == 3) dispatch_p_gather<3>(c, integrate, f_bead, f_sys, all_beads(c));
@@ -1556,10 +1619,16 @@ int tild_density_planar(tild_ctx* c, int s, float* dst, cudaStream_t st) {
 const float2* tild_half_spectra(tild_ctx* c, int s) {
   const SysHost& h = c->sys[s];
   const SysDev& d = c->h_sys[s];
+  Bucket& b = c->buckets[h.bucket];
+  if (!b.spectra) {  // of every system of the shape, from the densities that the last evaluation stored
+    if (exec_forward(c, b)) return nullptr;
+    b.spectra = true;
+  }
   if (!d.fwd_packed) return reinterpret_cast<const float2*>(c->rhok) + h.spec0;
   float2* half = reinterpret_cast<float2*>(c->gk) + h.spec0;
   k_unpack_half<<<nblk(h.g.Mh, 256), 256, 0, c->stream>>>(reinterpret_cast<const float2*>(c->rhok) + d.rkp0, half,
                                                            (h.T + h.C) / 2, h.g, h.D);
   c->launches++;
+  if (tild_check(c, cudaGetLastError(), "unpack spectra")) return nullptr;
   return half;
 }

@@ -290,6 +290,7 @@ int tild_build_tables(tild_ctx* c, int si) {
     k_charge_table<<<nblk(g.Mh, 256), 256, 0, st>>>(c->ctab + h.ctab0, g, D, h.cfg.bjerrum, h.cfg.smearing, ref, invM);
     c->launches++;
   }
+  if (rc == TILD_OK) rc = tild_fft_tables(c, si);
   for (const FieldK& fk : c->fields) {
     if (fk.sys != si || rc != TILD_OK) continue;
     const tild_pair_style& ps = h.cfg.styles[fk.cfg_index];
