@@ -772,13 +772,14 @@ int run_steps(tild_ctx* c, int n) {
       else if (n >= kMinGraphSteps) L = std::min(n, len);
     }
     if (L == 0) {
-      c->write_rho = n == 1;  // only the last step's densities can be read
+      c->last_of_call = n == 1;
       int rc = tild_run_forces(c, true, nullptr, -1);
-      c->write_rho = true;
+      c->last_of_call = true;
       if (rc) return rc;
       n -= 1;
       continue;
     }
+    if (tild_advance_steps(c)) return TILD_ERR_CUDA;  // graphs start from advanced counters
     if (L == len && aligned) c->steps_since_sort = c->sort_interval;  // a whole period starts with a sort
     const void* p0 = c->pos[0];
     const int cur = c->cur;
@@ -812,10 +813,10 @@ int run_steps(tild_ctx* c, int n) {
       return TILD_ERR_CUDA;
     int rc = TILD_OK;
     for (int k = 0; k < L && !rc; k++) {
-      c->write_rho = k == L - 1;
+      c->last_of_call = k == L - 1;
       rc = tild_run_forces(c, true, nullptr, -1);
     }
-    c->write_rho = true;
+    c->last_of_call = true;
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
     if (rc) {

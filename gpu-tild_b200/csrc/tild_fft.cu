@@ -191,23 +191,25 @@ __device__ __forceinline__ void with_radix(int R, F&& f) {
 
 __device__ __forceinline__ float2 swapped(float2 a) { return make_float2(a.y, a.x); }
 
-// Programmatic dependent launch: a pass lets the next one start as soon as all its CTAs run, and
-// touches what earlier kernels wrote (or still read) only after grid_wait().  Geometry, radices, unit
-// roots and multiplier tables are constant between host synchronisations, so they are fetched before.
-__device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;"); }
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // asynchronous 16-byte copies into shared memory
 __device__ __forceinline__ void copy_async16(void* smem, const void* global) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(global));
 }
 __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// A stride as an opaque value: its multiples are computed where they are used.  Hoisted out of the
+// (mostly single-trip) item loops, 15 of them per radix-16 access pattern spill (x forward at 128^3:
+// 22.7 against 15.9 us).
+__device__ __forceinline__ int here(int v) {
+  asm volatile("" : "+r"(v));
+  return v;
+}
+
 // An address that advances by a 32-bit byte step: one wide multiply-add per access.
 struct Run {
   char* p;
   unsigned step;
-  __device__ __forceinline__ Run(const void* at, unsigned bytes) : p((char*)at), step(bytes) {}
+  __device__ __forceinline__ Run(const void* at, unsigned bytes) : p((char*)at), step(here(bytes)) {}
   __device__ __forceinline__ float2& operator[](int k) const {
     return *reinterpret_cast<float2*>(p + (unsigned long long)step * (unsigned)k);
   }
@@ -293,19 +295,24 @@ struct FastDiv {
   __device__ __forceinline__ int div(int v) const { return d == 1 ? v : (int)__umulhi((unsigned)v, m); }
 };
 
-// Second stage by threads tid of nthreads: q counts (line, k1) combinations; src(q) is the first of its R2 values, `stride` their
-// distance; dst(q) is indexed by k2 for the results; put(dst, k2, value).
-template <class Src, class Dst, class Put>
-__device__ __forceinline__ void second_stage(int tid, int nthreads, int nq, int R1, int R2, int stride, const float2* __restrict__ tw,
-                                             Src&& src, Dst&& dst, Put&& put) {
-  if (R2 <= 16) {
+// Second stage by threads tid of nthreads: q counts (line, k1) combinations; src(q) is the first of its
+// R2 values, `stride` their distance; dst(q) is indexed by k2 for the results; put(dst, k2, value).
+// DIRECT: some system of the launch has R2 > 16.  Kernels without it are separate: the direct
+// transform's accumulators cost the radix stages beside it registers (128^3 z pass 36.7 against 33 us).  Only the x forward pass has one kernel
+// for both: it came out slower without (22 against 16.5 us).
+template <bool DIRECT, class Src, class Dst, class Put>
+__device__ __forceinline__ void second_stage(int tid, int nthreads, int nq, int R1, int R2, int stride,
+                                             const float2* __restrict__ tw, Src&& src, Dst&& dst, Put&& put) {
+  if (!DIRECT || R2 <= 16) {
     with_radix(R2, [&](auto rc) {
       constexpr int R = decltype(rc)::value;
+#pragma unroll 1
       for (int q = tid; q < nq; q += nthreads) {
         const float2* e = src(q);
+        const int pitch = here(stride);
         float2 v[R];
 #pragma unroll
-        for (int n = 0; n < R; n++) v[n] = e[n * stride];
+        for (int n = 0; n < R; n++) v[n] = e[n * pitch];
         dft<R>(v);
         const auto d = dst(q);
 #pragma unroll
@@ -318,6 +325,7 @@ __device__ __forceinline__ void second_stage(int tid, int nthreads, int nq, int 
     auto groups = [&](auto kc) {
       constexpr int K = decltype(kc)::value;
       const int ng = ((R2 + 1) / 2 + K - 1) / K;
+#pragma unroll 1
       for (int i = tid; i < nq * ng; i += nthreads) {
         const int gr = dq.div(i), q = i - gr * nq;
         const auto d = dst(q);
@@ -354,7 +362,7 @@ __host__ __device__ inline int rows_per_cta(int nx, int points) {
 __global__ void __launch_bounds__(kThreads, kMinCtas) k_fft_x_fwd(unsigned long long* __restrict__ fx, float* __restrict__ rho,
                                                    float2* __restrict__ zk, const float2* __restrict__ twid,
                                                    const int2* __restrict__ blocks, const SysDev* __restrict__ sysd,
-                                                   int D, int points, int write_rho, int blk_off) {
+                                                   int D, int points, int write_rho, int ahead, int blk_off) {
   extern __shared__ __align__(16) float2 ex[];
   const int2 bk = blocks[blockIdx.x + blk_off];
   const SysDev& sd = sysd[bk.x];
@@ -365,13 +373,14 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) k_fft_x_fwd(unsigned long 
   const int p = bk.y / tiles, row0 = (bk.y - p * tiles) * LT, nl = min(LT, rows - row0);
   const bool two = 2 * p + 1 < sd.T + sd.C, paired = sd.fwd_packed;
   unsigned long long* a = fx + sd.grid0 + 2 * (long long)p * g.M + (long long)row0 * g.nx;
-  unsigned long long* b = a + g.M;
   float* ra = rho + sd.grid0 + 2 * (long long)p * g.M;
   float2* rp = reinterpret_cast<float2*>(ra) + (long long)row0 * g.nx;
   ra += (long long)row0 * g.nx;
   grid_launch_next();
   grid_wait();
-  const bool act = sd.active;
+  const bool act = active_at(*after_wait(&sd), ahead);
+  a = after_wait(a);
+  unsigned long long* b = a + g.M;
   // the rows are one run of the grid: coalesced loads, kXBatch of each channel in flight per thread
   float2* in = ex + LT * R1 * R2p;
   const int npt = nl * g.nx;
@@ -411,23 +420,25 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) k_fft_x_fwd(unsigned long 
   const FastDiv dj(R2);
   with_radix(R1, [&](auto rc) {
     constexpr int R = decltype(rc)::value;
+#pragma unroll 1
     for (int i = threadIdx.x; i < nl * R2; i += kThreads) {
       const int line = dj.div(i), j = i - line * R2;
       const float2* s = in + line * g.nx + j;
+      const int from = here(R2), to = here(R2p);
       float2 v[R];
 #pragma unroll
-      for (int n = 0; n < R; n++) v[n] = s[n * R2];
+      for (int n = 0; n < R; n++) v[n] = s[n * from];
       dft_twiddle_rows<R>(v, j, R2, twr);
       float2* e = ex + line * R * R2p + j;
 #pragma unroll
-      for (int k = 0; k < R; k++) e[k * R2p] = v[k];
+      for (int k = 0; k < R; k++) e[k * to] = v[k];
     }
   });
   __syncthreads();
   float2* z = zk + sd.zk0 + (long long)p * g.M + (long long)row0 * g.nx;
   const FastDiv dk(R1);
   const unsigned step = R1 * sizeof(float2);
-  second_stage(threadIdx.x, kThreads, nl * R1, R1, R2, 1, tw, [&](int q) { return ex + q * R2p; },
+  second_stage<true>(threadIdx.x, kThreads, nl * R1, R1, R2, 1, tw, [&](int q) { return ex + q * R2p; },
                [&](int q) {
                  const int line = dk.div(q);
                  return Run(z + line * g.nx + (q - line * R1), step);
@@ -438,9 +449,10 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) k_fft_x_fwd(unsigned long 
 // ---- y forward, in place -------------------------------------------------------------------------
 // A CTA takes kColsFwd consecutive columns (x fastest, then z); lanes along the columns.  Past the
 // last column the last one is transformed again and not stored.
+template <bool DIRECT>
 __global__ void __launch_bounds__(kThreads, kMinCtas) k_fft_y_fwd(float2* __restrict__ zk, const float2* __restrict__ twid,
                                                    const int2* __restrict__ blocks, const SysDev* __restrict__ sysd,
-                                                   int blk_off) {
+                                                   int ahead, int blk_off) {
   extern __shared__ __align__(16) float2 ex[];
   constexpr int LT = kColsFwd;
   const int2 bk = blocks[blockIdx.x + blk_off];
@@ -456,9 +468,11 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) k_fft_y_fwd(float2* __rest
   char* z = reinterpret_cast<char*>(zk + sd.zk0 + (long long)p * g.M + (long long)cz * g.nx * g.ny + (c - cz * g.nx));
   grid_launch_next();
   grid_wait();
-  if (!sd.active) return;
+  if (!active_at(*after_wait(&sd), ahead)) return;
+  z = after_wait(z);
   with_radix(R1, [&](auto rc) {
     constexpr int R = decltype(rc)::value;
+#pragma unroll 1
     for (int j = threadIdx.x / LT; j < R2; j += kThreads / LT) {
       const Run s(z + j * row, R2 * row);
       float2 v[R];
@@ -471,7 +485,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) k_fft_y_fwd(float2* __rest
     }
   });
   __syncthreads();
-  second_stage(threadIdx.x, kThreads, R1 * LT, R1, R2, R1 * LT, tw, [&](int q) { return ex + q; },
+  second_stage<DIRECT>(threadIdx.x, kThreads, R1 * LT, R1, R2, R1 * LT, tw, [&](int q) { return ex + q; },
                [&](int q) { return Run(z + (q / LT) * row, R1 * row); },
                [&](const Run& d, int k2, float2 v) {
                  if (ok) d[k2] = v;
@@ -561,11 +575,12 @@ __device__ __forceinline__ void multiply_tile(int T, U&& multiplier, Spec&& spec
 // a pair's spectra apart needs: X_2p(k) = (Z(k) + conj Z(-k)) / 2, X_2p+1 = (Z(k) - conj Z(-k)) / 2i.
 // A CTA takes kColsZ columns and their mirrors (as many further lines) of every pair of a system.
 // Its halves transform two pairs at once, and the two inverse fields of a pair.
-__global__ void __launch_bounds__(kThreadsZ, kMinCtasZ) k_fft_z_kmul(const float2* __restrict__ zk, float2* __restrict__ gk,
+template <bool DIRECT>
+__global__ void __launch_bounds__(kThreadsZ, kMinCtasZ) k_fft_z_kmul(const float2* zk, float2* __restrict__ gk,
                                                     const float* __restrict__ ztab, const float* __restrict__ utab_all,
                                                     const float* __restrict__ ctab_all, const float* __restrict__ kd_all,
                                                     const float2* __restrict__ twid, const int2* __restrict__ blocks,
-                                                    const SysDev* __restrict__ sysd, int D, int integrate, int blk_off) {
+                                                    const SysDev* __restrict__ sysd, int D, int integrate, int ahead, int blk_off) {
   extern __shared__ __align__(16) float2 sm[];
   __shared__ float s_scale[kTilePairs];  // ramp factor of each type pair
   constexpr int LT = kColsZ, LL = 2 * LT;
@@ -600,9 +615,11 @@ __global__ void __launch_bounds__(kThreadsZ, kMinCtasZ) k_fft_z_kmul(const float
   const long long at = mirror ? (long long)my * nx + mx : (long long)ky * nx + kx;
   const unsigned pl = (unsigned)(nx * ny * (int)sizeof(float2));
   grid_wait();
-  grid_launch_next();  // only now: whatever starts early from here on finds the last step's kernels done
-  const long long est = sd.step + (integrate ? 1 : 0);
-  if (!sd.active) return;
+  grid_launch_next();  // only now: what starts early from here on (the gather) finds the last step's kernels done
+  const SysDev* now = after_wait(&sd);
+  const long long est = now->step + ahead + (integrate ? 1 : 0);
+  if (!active_at(*now, ahead)) return;
+  zk = after_wait(zk);
   if (tile && threadIdx.x < nu) s_scale[threadIdx.x] = sd.zramp[threadIdx.x] < 0 ? 1.f : ramp_ratio(sd, sd.zramp[threadIdx.x], est);
   for (int p0 = 0; p0 < np; p0 += 2) {
     const int p = p0 + half;
@@ -612,6 +629,7 @@ __global__ void __launch_bounds__(kThreadsZ, kMinCtasZ) k_fft_z_kmul(const float
       const char* z = reinterpret_cast<const char*>(zk + sd.zk0 + (long long)p * g.M + at);
       with_radix(R1, [&](auto rc) {
         constexpr int R = decltype(rc)::value;
+#pragma unroll 1
         for (int j = ht / LL; j < R2; j += kThreadsZ / 2 / LL) {
           const Run s(z + (unsigned long long)pl * (unsigned)j, pl * R2);
           float2 v[R];
@@ -627,7 +645,7 @@ __global__ void __launch_bounds__(kThreadsZ, kMinCtasZ) k_fft_z_kmul(const float
     __syncthreads();
     float2* pz = pb + p * exn;
     if (on)
-      second_stage(ht, kThreadsZ / 2, R1 * LL, R1, R2, R1 * LL, tw, [&](int q) { return ex + q; },
+      second_stage<DIRECT>(ht, kThreadsZ / 2, R1 * LL, R1, R2, R1 * LL, tw, [&](int q) { return ex + q; },
                    [&](int q) { return pz + q; },
                    [&](float2* d, int k2, float2 v) { d[k2 * (R1 * LL)] = v; });
   }
@@ -693,9 +711,10 @@ __global__ void __launch_bounds__(kThreadsZ, kMinCtasZ) k_fft_z_kmul(const float
     __syncthreads();
     with_radix(R1, [&](auto rc) {
       constexpr int R = decltype(rc)::value;
+#pragma unroll 1
       for (int j = ht / LL; j < R2; j += kThreadsZ / 2 / LL) {
         const float2* s = pz + j * LL;
-        const int step = R2 * LL;
+        const int step = here(R2 * LL);
         float2 v[R];
 #pragma unroll
         for (int n = 0; n < R; n++) v[n] = swapped(s[n * step]);
@@ -713,7 +732,7 @@ __global__ void __launch_bounds__(kThreadsZ, kMinCtasZ) k_fft_z_kmul(const float
       }
     });
     __syncthreads();
-    second_stage(ht, kThreadsZ / 2, R1 * LL, R1, R2, R1 * LL, tw, [&](int q) { return ex + q; },
+    second_stage<DIRECT>(ht, kThreadsZ / 2, R1 * LL, R1, R2, R1 * LL, tw, [&](int q) { return ex + q; },
                  [&](int q) { return Run(out + (unsigned long long)pl * (q / LL), pl * R1); },
                  [&](const Run& d, int k2, float2 v) {
                    if (store) d[k2] = D == 2 && !f ? make_float2(kx_f * v.x, -kx_f * v.y) : swapped(v);
@@ -730,10 +749,10 @@ struct Field {
 // LT = 8: the CTA's threads transform the three fields of 8 columns at once (small grids: the most
 // threads at work).  LT = 16: 128-byte runs, one field after another (large grids: 64-byte runs at
 // power-of-two strides cost twice the L1 wavefronts).
-template <int LT>
+template <int LT, bool DIRECT>
 __global__ void __launch_bounds__(LT == 8 ? 192 : 128, LT == 8 ? 5 : 8)
     k_fft_y_inv(float2* __restrict__ gk, const float* __restrict__ kd_all, const float2* __restrict__ twid,
-                const int2* __restrict__ blocks, const SysDev* __restrict__ sysd, int blk_off) {
+                const int2* __restrict__ blocks, const SysDev* __restrict__ sysd, int ahead, int blk_off) {
   extern __shared__ __align__(16) float2 ex[];
   constexpr int THREADS = LT == 8 ? 192 : 128, NF = LT == 8 ? 3 : 1;  // NF fields at once
   const int2 bk = blocks[blockIdx.x + blk_off];
@@ -754,12 +773,14 @@ __global__ void __launch_bounds__(LT == 8 ? 192 : 128, LT == 8 ? 5 : 8)
   const FastDiv dr(R2), df(nq);
   grid_launch_next();
   grid_wait();
-  if (!sd.active) return;
+  if (!active_at(*after_wait(&sd), ahead)) return;
+  z = after_wait(z);
   // P's y derivative first: P itself is overwritten by its x derivative
   for (int f0 = 0; f0 < 3; f0 += NF) {
     if (f0) __syncthreads();
     with_radix(R1, [&](auto rc) {
       constexpr int R = decltype(rc)::value;
+#pragma unroll 1
       for (int i = threadIdx.x / LT; i < NF * R2; i += THREADS / LT) {
         const int fi = NF == 1 ? 0 : dr.div(i), j = i - fi * R2, f = f0 + fi;  // 0: y, 1: x, 2: z derivative
         const Run s(z + (f == 2 ? 2 * field : 0) + j * row, R2 * row);
@@ -780,7 +801,7 @@ __global__ void __launch_bounds__(LT == 8 ? 192 : 128, LT == 8 ? 5 : 8)
       }
     });
     __syncthreads();
-    second_stage(threadIdx.x, THREADS, NF * nq, R1, R2, R1p * LT, tw,
+    second_stage<DIRECT>(threadIdx.x, THREADS, NF * nq, R1, R2, R1p * LT, tw,
                  [&](int q) {
                    const int fi = NF == 1 ? 0 : df.div(q);
                    return ex + fi * exn + (q - fi * nq);
@@ -799,9 +820,10 @@ __global__ void __launch_bounds__(LT == 8 ? 192 : 128, LT == 8 ? 5 : 8)
 // A CTA takes consecutive rows of one pair in all D fields; the second stage leaves its results in
 // shared memory and the rows are written as float4 nodes (real parts to channel 2p, imaginary parts
 // to 2p + 1), lanes along x.
+template <bool DIRECT>
 __global__ void __launch_bounds__(kThreadsX, kMinCtasX) k_fft_x_inv(const float2* __restrict__ gk, float4* __restrict__ g4_all,
                                                    const float2* __restrict__ twid, const int2* __restrict__ blocks,
-                                                   const SysDev* __restrict__ sysd, int D, int points, int layout, int blk_off) {
+                                                   const SysDev* __restrict__ sysd, int D, int points, int layout, int ahead, int blk_off) {
   extern __shared__ __align__(16) float2 ex[];
   __shared__ int s_row[32];  // node offset of each row
   const int2 bk = blocks[blockIdx.x + blk_off];
@@ -821,9 +843,11 @@ __global__ void __launch_bounds__(kThreadsX, kMinCtasX) k_fft_x_inv(const float2
   }
   grid_launch_next();
   grid_wait();
-  if (!sd.active) return;
+  if (!active_at(*after_wait(&sd), ahead)) return;
+  src = after_wait(src);
   with_radix(R1, [&](auto rc) {
     constexpr int R = decltype(rc)::value;
+#pragma unroll 1
     for (int i = threadIdx.x; i < D * nl * R2; i += kThreadsX) {
       const int fl = dj.div(i), j = i - fl * R2, f = dl.div(fl), line = fl - f * nl;
       const Run s(src + f * g.M + line * nx + j, R2 * sizeof(float2));
@@ -832,8 +856,9 @@ __global__ void __launch_bounds__(kThreadsX, kMinCtasX) k_fft_x_inv(const float2
       for (int n = 0; n < R; n++) v[n] = swapped(s[n]);
       dft_twiddle_rows<R>(v, j, R2, twr);
       float2* e = ex + f * exn + line * R * R2p + j;
+      const int to = here(R2p);
 #pragma unroll
-      for (int k = 0; k < R; k++) e[k * R2p] = v[k];
+      for (int k = 0; k < R; k++) e[k * to] = v[k];
     }
   });
   __syncthreads();
@@ -853,9 +878,10 @@ __global__ void __launch_bounds__(kThreadsX, kMinCtasX) k_fft_x_inv(const float2
     const int f = df.div(q);
     return f * exn + (q - f * nq) * R2p;
   };
-  second_stage(threadIdx.x, kThreadsX, D * nq, R1, R2, 1, tw, [&](int q) { return ex + slot(q); },
+  second_stage<DIRECT>(threadIdx.x, kThreadsX, D * nq, R1, R2, 1, tw, [&](int q) { return ex + slot(q); },
                [&](int q) { return res + slot(q); }, [](float2* d, int k2, float2 v) { d[k2] = v; });
   __syncthreads();
+#pragma unroll 1
   for (int i = threadIdx.x; i < nl * nx; i += kThreadsX) {
     const int k2 = df.div(i), q = i - k2 * nq, line = dk.div(q), x = q - line * R1 + R1 * k2;
     const float2* r = res + q * R2p + k2;
@@ -924,29 +950,6 @@ size_t z_smem(int nz, int T, int C) {
   return (2 + np) * 4 * line + (np > 1 || nu > 4 ? nu * line : 0);
 }
 
-// A pass may start while the kernel before it still runs (grid_wait).  All passes ask for one split of
-// the SM's 228 KB: an SM that has to change its split between two kernels drains first, so the next
-// pass could not start early there (40^3, 40,000 beads: 36.3 us a step with one split, 46.4 with the
-// driver's choice for each pass, 39 without the early starts).  60 per cent hold the CTAs that the
-// registers allow and leave L1 to the unit roots (96^3, 4 channels: 133 us a step against 139 at 100).
-constexpr int kCarveout = 60;
-template <class... P, class... A>
-void launch_pass(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  at[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-  at[1].val.sharedMemCarveout = kCarveout;
-  cfg.numAttrs = 2;
-  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
-}
-
 template <class K>
 bool allow_smem(K* k) {
   const void* f = reinterpret_cast<const void*>(k);
@@ -998,6 +1001,9 @@ int tild_fft_setup(tild_ctx* c) {
           const int N = g.nx[a];
           int r1, r2;
           split_length(N, &r1, &r2);
+          const int axis = a == D - 1 ? 2 : a;  // of the passes: x, y, z
+          b.fft_direct[axis] = b.fft_direct[axis] || r2 > 16;
+          c->fft_direct[axis] = c->fft_direct[axis] || r2 > 16;
           d.fft_r1[a] = (short)r1;
           d.fft_r2[a] = (short)r2;
           size_t k = 0;
@@ -1054,8 +1060,10 @@ int tild_fft_setup(tild_ctx* c) {
     if (tild_check(c, cudaMemcpyAsync(c->fft_pass[k].blocks, tab[k].data(), sizeof(int2) * tab[k].size(), cudaMemcpyHostToDevice, c->stream), "transform blocks"))
       return TILD_ERR_CUDA;
   }
-  const bool okattr = allow_smem(k_fft_x_fwd) && allow_smem(k_fft_y_fwd) && allow_smem(k_fft_z_kmul) &&
-                      allow_smem(k_fft_y_inv<8>) && allow_smem(k_fft_y_inv<16>) && allow_smem(k_fft_x_inv);
+  auto both = [](auto* regular, auto* direct) { return allow_smem(regular) && allow_smem(direct); };
+  const bool okattr = allow_smem(k_fft_x_fwd) && both(k_fft_y_fwd<false>, k_fft_y_fwd<true>) &&
+                      both(k_fft_z_kmul<false>, k_fft_z_kmul<true>) && both(k_fft_y_inv<8, false>, k_fft_y_inv<8, true>) &&
+                      both(k_fft_y_inv<16, false>, k_fft_y_inv<16, true>) && both(k_fft_x_inv<false>, k_fft_x_inv<true>);
   if (!okattr) {
     c->err = "shared memory of the transform passes";
     return TILD_ERR_CUDA;
@@ -1105,29 +1113,30 @@ int tild_fft_run(tild_ctx* c, const Bucket* b, bool integrate, bool active, cuda
   float2* zk = reinterpret_cast<float2*>(c->rhok);
   float2* gk = reinterpret_cast<float2*>(c->gk);
   const auto* pa = c->fft_pass;
-  const int wr = c->write_rho || !c->fields.empty();
+  const int wr = !integrate || c->last_of_call || !c->fields.empty(), ahead = c->ahead;
+  const bool* dir = b ? b->fft_direct : c->fft_direct;
   if (!b) tild_mark(c, STAGE_ZERO);
-  launch_pass(k_fft_x_fwd, n[0], kThreads, pa[0].smem, st, c->rho_fx, c->rho, zk, c->fft_twid, pa[0].blocks, c->d_sys, c->D, c->fft_points, wr, off[0]);
+  tild_launch_early(k_fft_x_fwd, n[0], kThreads, pa[0].smem, kCarveout, st, c->rho_fx, c->rho, zk, c->fft_twid, pa[0].blocks, c->d_sys, c->D, c->fft_points, wr, ahead, off[0]);
   c->launches++;
   if (!active) return tild_check(c, cudaGetLastError(), "grid passes");  // no system of the shape moves: densities only
   if (c->D == 3) {
     if (!b) tild_mark(c, STAGE_R2C);
-    launch_pass(k_fft_y_fwd, n[1], kThreads, pa[1].smem, st, zk, c->fft_twid, pa[1].blocks, c->d_sys, off[1]);
+    tild_launch_early(dir[1] ? k_fft_y_fwd<true> : k_fft_y_fwd<false>, n[1], kThreads, pa[1].smem, kCarveout, st, zk, c->fft_twid, pa[1].blocks, c->d_sys, ahead, off[1]);
     c->launches++;
   }
   if (!b) tild_mark(c, STAGE_KMUL);
-  launch_pass(k_fft_z_kmul, n[2], kThreadsZ, pa[2].smem, st, zk, gk, c->ztab, c->utab, c->ctab, c->kd, c->fft_twid, pa[2].blocks, c->d_sys,
-              c->D, (int)integrate, off[2]);
+  tild_launch_early(dir[2] ? k_fft_z_kmul<true> : k_fft_z_kmul<false>, n[2], kThreadsZ, pa[2].smem, kCarveout, st, zk, gk, c->ztab, c->utab, c->ctab, c->kd, c->fft_twid, pa[2].blocks, c->d_sys,
+              c->D, (int)integrate, ahead, off[2]);
   if (c->D == 3) {
     if (!b) tild_mark(c, STAGE_C2R);
     if (c->fft_wide)
-      launch_pass(k_fft_y_inv<16>, n[3], 128, pa[3].smem, st, gk, c->kd, c->fft_twid, pa[3].blocks, c->d_sys, off[3]);
+      tild_launch_early(dir[1] ? k_fft_y_inv<16, true> : k_fft_y_inv<16, false>, n[3], 128, pa[3].smem, kCarveout, st, gk, c->kd, c->fft_twid, pa[3].blocks, c->d_sys, ahead, off[3]);
     else
-      launch_pass(k_fft_y_inv<8>, n[3], 192, pa[3].smem, st, gk, c->kd, c->fft_twid, pa[3].blocks, c->d_sys, off[3]);
+      tild_launch_early(dir[1] ? k_fft_y_inv<8, true> : k_fft_y_inv<8, false>, n[3], 192, pa[3].smem, kCarveout, st, gk, c->kd, c->fft_twid, pa[3].blocks, c->d_sys, ahead, off[3]);
     c->launches++;
   }
   if (!b) tild_mark(c, STAGE_INTERLEAVE);
-  launch_pass(k_fft_x_inv, n[4], kThreadsX, pa[4].smem, st, gk, c->g4, c->fft_twid, pa[4].blocks, c->d_sys, c->D, c->fft_points, c->field_layout, off[4]);
+  tild_launch_early(dir[0] ? k_fft_x_inv<true> : k_fft_x_inv<false>, n[4], kThreadsX, pa[4].smem, kCarveout, st, gk, c->g4, c->fft_twid, pa[4].blocks, c->d_sys, c->D, c->fft_points, c->field_layout, ahead, off[4]);
   c->launches += 2;
   return tild_check(c, cudaGetLastError(), "grid passes");
 }

@@ -88,6 +88,12 @@ struct SysDev {
   float bond_k[TILD_MAX_BOND_TYPES], bond_req[TILD_MAX_BOND_TYPES];
 };
 
+// A system's state `ahead` steps after the device counters were last advanced: whether it still moves,
+// and its completed steps.
+__device__ __forceinline__ bool active_at(const SysDev& sd, int ahead) {
+  return sd.active && (sd.stop_at < 0 || sd.step + ahead < sd.stop_at);
+}
+
 struct FieldK {     // one fieldphase style
   int sys, a, b;
   int cfg_index;
@@ -129,6 +135,7 @@ struct Bucket {     // systems sharing one grid shape: one batched R2C plan and 
   bool own = false;
   bool spectra = false;                  // rhok holds the library spectra of the last force evaluation
   int fft_blk0[5] = {0}, fft_nblk[5] = {0};
+  bool fft_direct[3] = {false, false, false};  // the x, y, z axis takes the direct transform
   int cta_spec0 = 0, n_cta_spec = 0;     // the shape's range of spectrum blocks (k-space multiply)
   int cta_grid0 = 0, n_cta_grid = 0;     // and of grid blocks (interleave)
   int cta_bead0 = 0, n_cta_bead = 0;     // and of particle blocks (spread, gather)
@@ -161,9 +168,14 @@ struct tild_ctx {
   FftPass fft_pass[5];                   // x, y forward, z with the multiply, y, x inverse
   float2* fft_twid = nullptr;
   float* ztab = nullptr;                 // multipliers in the z pass's order
+  bool fft_direct[3] = {false, false, false};  // of some shape
   bool fft_wide = false;                 // 16 columns per CTA in the y inverse pass
   int fft_points = 1024;                 // points per field of an x pass's CTA
-  bool write_rho = true;                 // the next force evaluation stores the float densities
+  // The next integrating step is the last of its call: it stores the float densities (only they can be
+  // read) and advances the device's step counters by the call's steps.  Until then kernels count
+  // `ahead` steps beyond them.
+  bool last_of_call = true;
+  int ahead = 0;
   int D = 3, P = 1;
   int nsys = 1;
   std::vector<SysHost> sys;
@@ -214,7 +226,7 @@ struct tild_ctx {
   double* red = nullptr;
   int red_cap = 0;
   float* xfer = nullptr;                 // staging for host transfers, >= 3 * max ns floats
-  int* d_status = nullptr;
+  int* d_status = nullptr;               // [0] status word, [1] input check flag
 
   // spatial sort (tild_sort.cu)
   unsigned* sort_keys = nullptr;
@@ -309,6 +321,44 @@ inline void tild_mark(tild_ctx* c, int stage) {
   c->prof_ev.push_back(e);
   c->prof_stage.push_back(stage);
 }
+
+// ---- programmatic dependent launch -----------------------------------------------------------
+// A kernel launched with tild_launch_early may start while the kernel before it in the stream still
+// runs, once all CTAs of that kernel have called grid_launch_next() or ended.  It touches what earlier
+// kernels write or still read only after grid_wait(), through pointers passed through after_wait()
+// (the compiler may move read-only loads across the wait otherwise).
+__device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class T>
+__device__ __forceinline__ T* after_wait(T* p) {
+  size_t g = __cvta_generic_to_global(p);  // a global address still: generic loads cost the passes 7 %
+  asm volatile("" : "+l"(g)::"memory");
+  return static_cast<T*>(__cvta_global_to_generic(g));
+}
+// carveout: per cent of the SM's 228 KB preferred as shared memory (-1: the function's own setting)
+template <class... P, class... A>
+inline void tild_launch_early(void (*kernel)(P...), int grid, int threads, size_t smem, int carveout, cudaStream_t st,
+                              A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  at[1].val.sharedMemCarveout = carveout < 0 ? 0 : carveout;
+  cfg.attrs = at;
+  cfg.numAttrs = carveout < 0 ? 1 : 2;
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+// One shared-memory split for the passes of a step: an SM that has to change its split between two
+// kernels drains first, so the next one could not start early there (40^3, 40,000 beads: 36.3 us a step
+// with one split for the grid passes, 46.4 with the driver's choice for each, 39 without early starts).
+// 60 per cent hold the CTAs that the registers allow and leave L1 to the unit roots (96^3, 4 channels:
+// 133 us a step against 139 at 100).
+constexpr int kCarveout = 60;
 
 // ---- small helpers -----------------------------------------------------------------------
 // Per-channel storage of the float4 force field: room for the brick layout (3D: 4x4x4 bricks,
@@ -452,6 +502,7 @@ __host__ __device__ inline float ramp_ratio(const SysDev& d, int k, long long st
 // ---- host-side entry points between translation units ------------------------------------
 int tild_build_tables(tild_ctx* c, int s);            // tild_tables.cu
 int tild_run_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys);   // tild_step.cu
+int tild_advance_steps(tild_ctx* c);
 int tild_finish_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys, bool interleaved, bool gathered);
 int tild_density_planar(tild_ctx* c, int s, float* dst, cudaStream_t st);                 // tild_step.cu
 const float2* tild_half_spectra(tild_ctx* c, int s);                                     // tild_step.cu

@@ -421,16 +421,16 @@ __global__ void __launch_bounds__(256) k_kmul(const float2* __restrict__ rhok_al
                                              const float* __restrict__ utab_all, const float* __restrict__ ctab_all,
                                              const float* __restrict__ kd_all, const int* __restrict__ cta_sys,
                                              const int* __restrict__ blk0, const SysDev* __restrict__ sysd,
-                                             int integrate, int blk_off) {
+                                             int integrate, int ahead, int blk_off) {
   const int blk = blockIdx.x + blk_off;
   const int s = cta_sys[blk];
   const SysDev& sd = sysd[s];
-  if (!sd.active) return;  // one system per CTA; inactive systems are not gathered
+  if (!active_at(sd, ahead)) return;  // one system per CTA; inactive systems are not gathered
   // per-CTA style table: the CTA covers one system
   __shared__ float s_scale[TILD_MAX_STYLES];
   __shared__ int s_ab[TILD_MAX_STYLES];
   __shared__ int s_nfft;
-  const long long est = sd.step + (integrate ? 1 : 0);
+  const long long est = sd.step + ahead + (integrate ? 1 : 0);
   if (threadIdx.x < TILD_MAX_STYLES && threadIdx.x < sd.nfft) {
     s_scale[threadIdx.x] = ramp_ratio(sd, threadIdx.x, est);
     s_ab[threadIdx.x] = sd.sa[threadIdx.x] | (sd.sb[threadIdx.x] << 8);
@@ -567,11 +567,11 @@ __global__ void k_fieldphase_apply(float* __restrict__ gfield, const float* __re
 template <int D>
 __global__ void k_interleave(const float* __restrict__ planar_all, const float2* __restrict__ pairs_all,
                              float4* __restrict__ g4_all, const int* __restrict__ cta_sys, const int* __restrict__ blk0,
-                             const SysDev* __restrict__ sysd, int layout, int blk_off) {
+                             const SysDev* __restrict__ sysd, int layout, int ahead, int blk_off) {
   const int blk = blockIdx.x + blk_off;
   const int s = cta_sys[blk];
   const SysDev& sd = sysd[s];
-  if (!sd.active) return;  // inactive systems are not gathered
+  if (!active_at(sd, ahead)) return;  // inactive systems are not gathered
   const Geom& g = sd.g;
   const long long M = g.M;
   const long long m = (long long)(blk - blk0[s]) * blockDim.x + threadIdx.x;
@@ -785,7 +785,7 @@ __device__ __forceinline__ void bead_epilogue(int i, const float4& p, int t, flo
                                               const float4 (&pj)[3], int bid, const float4& po,
                                               float* __restrict__ noise, float4* __restrict__ pos_io,
                                               float* __restrict__ f_out, int f_sys, int s,
-                                              curandStateXORWOW_t* __restrict__ xw) {
+                                              curandStateXORWOW_t* __restrict__ xw, int ahead) {
   // bonds
 #pragma unroll
   for (int bb = 0; bb < 3; bb++) {
@@ -815,7 +815,7 @@ __device__ __forceinline__ void bead_epilogue(int i, const float4& p, int t, flo
   if (!INTEG) return;
   // integrators in input order (integrator.cu:24-39 is called for each in turn)
   const int mask = sd.type_mask[t];
-  const long long est = sd.step + 1;
+  const long long est = sd.step + ahead + 1;
   float xo[3] = {po.x, po.y, po.z};
   float on[3] = {0.f, 0.f, 0.f};
   bool any_gjf = false;
@@ -881,7 +881,7 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : (P >= 3 ? 4 : (P >= 2 ? 3 :
     const int* __restrict__ bead_id, const int* __restrict__ bond_nbr, const int* __restrict__ bond_info,
     const float* __restrict__ charge, const float4* __restrict__ g4_all, const int* __restrict__ cta_sys,
     const SysDev* __restrict__ sysd, float* __restrict__ f_out, int f_sys, curandStateXORWOW_t* __restrict__ xw,
-    int layout, unsigned long long* __restrict__ rho_fx_all, int spread_cap, int* status, int blk_off) {
+    int layout, unsigned long long* __restrict__ rho_fx_all, int spread_cap, int* status, int ahead, int blk_off) {
   static_assert(SPR == 0 || INTEG, "only integrating launches spread ahead");
   const int s = cta_sys[blockIdx.x + blk_off];
   const SysDev& sd = sysd[s];
@@ -893,7 +893,7 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : (P >= 3 ? 4 : (P >= 2 ? 3 :
   const int C = sd.C;
   const float q = (CH && C && t != kPadType) ? charge[i] : 0.f;
   bool sp = false;  // x (after the update) is spread ahead
-  if (!sd.active) {  // one system per CTA: every thread takes this branch together
+  if (!active_at(sd, ahead)) {  // one system per CTA: every thread takes this branch together
     if (INTEG) pos_io[i] = p;  // inactive systems keep x_n through the buffer rotation
     if (SPR == 0) return;
     sp = t != kPadType && finite;  // held positions are spread too
@@ -930,7 +930,7 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : (P >= 3 ? 4 : (P >= 2 ? 3 :
       const int bid = bead_id[i];
       float4 po = make_float4(0.f, 0.f, 0.f, 0.f);
       if (INTEG) po = pos_io[i];
-      bead_epilogue<D, INTEG, XW>(i, p, t, x, f, sd, g, info, nb, pj, bid, po, noise, pos_io, f_out, f_sys, s, xw);
+      bead_epilogue<D, INTEG, XW>(i, p, t, x, f, sd, g, info, nb, pj, bid, po, noise, pos_io, f_out, f_sys, s, xw, ahead);
       if (SPR != 0) {
         sp = isfinite(x[0]) && isfinite(x[1]) && isfinite(x[2]);
         if (!sp) atomicOr(status, ST_NONFINITE_POS);
@@ -976,7 +976,7 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : (P >= 3 ? 4 : (P >= 2 ? 3 :
     const int bid = bead_id[i];
     float4 po = make_float4(0.f, 0.f, 0.f, 0.f);
     if (INTEG) po = pos_io[i];  // x_{n-1} (GJF xo)
-    bead_epilogue<D, INTEG, XW>(i, p, t, x, f, sd, g, info, nb, pj, bid, po, noise, pos_io, f_out, f_sys, s, xw);
+    bead_epilogue<D, INTEG, XW>(i, p, t, x, f, sd, g, info, nb, pj, bid, po, noise, pos_io, f_out, f_sys, s, xw, ahead);
     if (SPR != 0) {
       sp = isfinite(x[0]) && isfinite(x[1]) && (D == 2 || isfinite(x[2]));
       if (!sp) atomicOr(status, ST_NONFINITE_POS);
@@ -1026,7 +1026,7 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : 3)) k_gather_box(
     const int* __restrict__ bead_id, const int* __restrict__ bond_nbr, const int* __restrict__ bond_info,
     const float* __restrict__ charge, const float4* __restrict__ g4_all, const int* __restrict__ cta_sys,
     const SysDev* __restrict__ sysd, float* __restrict__ f_out, int f_sys, curandStateXORWOW_t* __restrict__ xw,
-    int box_cap, int* status, int blk_off) {
+    int box_cap, int* status, int ahead, int blk_off) {
   extern __shared__ float4 sbox[];
   __shared__ int s_g0[3], s_min[3], s_max[3];
   __shared__ int s_row[kMaxRows];
@@ -1034,7 +1034,7 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : 3)) k_gather_box(
   const SysDev& sd = sysd[s];
   const int i0 = (blockIdx.x + blk_off) * blockDim.x;
   const int i = i0 + threadIdx.x;
-  if (!sd.active) {  // one system per CTA: every thread leaves here together
+  if (!active_at(sd, ahead)) {  // one system per CTA: every thread leaves here together
     if (INTEG) pos_io[i] = pos_in[i];
     return;
   }
@@ -1168,17 +1168,18 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : 3)) k_gather_box(
     }
   }
   if (!ok) return;
-  bead_epilogue<D, INTEG, XW>(i, p, t, x, f, sd, g, info, nb, pj, bid, po, noise, pos_io, f_out, f_sys, s, xw);
+  bead_epilogue<D, INTEG, XW>(i, p, t, x, f, sd, g, info, nb, pj, bid, po, noise, pos_io, f_out, f_sys, s, xw, ahead);
 }
 
-// step counters advance on the device; a system whose counter reaches its stop step leaves the
-// active set here, so the next launches skip it without the host in the loop
-__global__ void k_advance_steps(SysDev* __restrict__ sysd, int nsys) {
+// n steps of every active system, on the device; a system whose counter reaches its stop step takes
+// the steps up to it and leaves the active set, so the next launches skip it without the host in the
+// loop.  Once a call, not once a step: the launch was 1.9 us of each step's path.
+__global__ void k_advance_steps(SysDev* __restrict__ sysd, int nsys, int n) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsys || !sysd[s].active) return;
-  const long long step = sysd[s].step + 1;
-  sysd[s].step = step;
-  if (sysd[s].stop_at >= 0 && step >= sysd[s].stop_at) sysd[s].active = 0;
+  const long long stop = sysd[s].stop_at, step = sysd[s].step + n;
+  sysd[s].step = stop >= 0 && step > stop ? stop : step;
+  if (stop >= 0 && step >= stop) sysd[s].active = 0;
 }
 
 // Order <= 1 always spreads directly; order >= 2 uses the shared box unless the tuner chose the
@@ -1230,7 +1231,7 @@ void launch_gather_k(tild_ctx* c, float* f_out, int f_sys, BeadRange r) {
     }
     k_gather_box<D, P, I, X, CH><<<r.n, kTile, sizeof(float4) * (size_t)c->gather_cap, r.st>>>(
         c->pos[c->cur], c->pos[c->cur ^ 1], c->noise, c->bead_id, c->bond_nbr, c->bond_info, c->charge, c->g4,
-        c->cta_bead, c->d_sys, f_out, f_sys, c->xorwow, c->gather_cap, c->d_status, r.off);
+        c->cta_bead, c->d_sys, f_out, f_sys, c->xorwow, c->gather_cap, c->d_status, c->ahead, r.off);
     return;
   }
   if constexpr (I) {
@@ -1247,7 +1248,7 @@ void launch_gather_k(tild_ctx* c, float* f_out, int f_sys, BeadRange r) {
           k_gather<D, P, I, X, CH, 1><<<r.n, kTile, sizeof(int) * (size_t)c->spread_cap, r.st>>>(
               c->pos[c->cur], c->pos[c->cur ^ 1], c->noise, c->bead_id, c->bond_nbr, c->bond_info, c->charge, c->g4,
               c->cta_bead, c->d_sys, f_out, f_sys, c->xorwow, c->field_layout, c->rho_fx, c->spread_cap,
-              c->d_status, r.off);
+              c->d_status, c->ahead, r.off);
           return;
         }
       }
@@ -1262,7 +1263,7 @@ void launch_gather_k(tild_ctx* c, float* f_out, int f_sys, BeadRange r) {
       }
       k_gather<D, P, I, X, CH, 2><<<r.n, kTile, 0, r.st>>>(  // spread ahead by global atomics
           c->pos[c->cur], c->pos[c->cur ^ 1], c->noise, c->bead_id, c->bond_nbr, c->bond_info, c->charge, c->g4,
-          c->cta_bead, c->d_sys, f_out, f_sys, c->xorwow, c->field_layout, c->rho_fx, 0, c->d_status, r.off);
+          c->cta_bead, c->d_sys, f_out, f_sys, c->xorwow, c->field_layout, c->rho_fx, 0, c->d_status, c->ahead, r.off);
       return;
     }
   }
@@ -1290,7 +1291,7 @@ void launch_gather_k(tild_ctx* c, float* f_out, int f_sys, BeadRange r) {
   }
   k_gather<D, P, I, X, CH, 0><<<r.n, kTile, 0, r.st>>>(
       c->pos[c->cur], c->pos[c->cur ^ 1], c->noise, c->bead_id, c->bond_nbr, c->bond_info, c->charge, c->g4,
-      c->cta_bead, c->d_sys, f_out, f_sys, c->xorwow, c->field_layout, nullptr, 0, c->d_status, r.off);
+      c->cta_bead, c->d_sys, f_out, f_sys, c->xorwow, c->field_layout, nullptr, 0, c->d_status, c->ahead, r.off);
 }
 
 template <int D, int P, bool I, bool X>
@@ -1339,10 +1340,10 @@ void launch_interleave(tild_ctx* c, cudaStream_t st, int off, int n) {
   int* blk0 = c->cta_grid + c->n_cta_grid;
   if (c->D == 3)
     k_interleave<3><<<n, 256, 0, st>>>(c->gfield, reinterpret_cast<const float2*>(c->gk), c->g4, c->cta_grid, blk0,
-                                       c->d_sys, c->field_layout, off);
+                                       c->d_sys, c->field_layout, c->ahead, off);
   else
     k_interleave<2><<<n, 256, 0, st>>>(c->gfield, reinterpret_cast<const float2*>(c->gk), c->g4, c->cta_grid, blk0,
-                                       c->d_sys, c->field_layout, off);
+                                       c->d_sys, c->field_layout, c->ahead, off);
 }
 
 // k-space multiply over spectrum blocks [off, off + n) (all of them by default) on stream st
@@ -1355,11 +1356,11 @@ void launch_kmul(tild_ctx* c, bool integ, cudaStream_t st = nullptr, int off = 0
   if (!st) st = c->stream;
   if (n == 0) return;
   switch (c->maxT) {
-    case 1: k_kmul<D, 1><<<n, 256, 0, st>>>(rk, gk, c->utab, c->ctab, c->kd, c->cta_spec, blk0, c->d_sys, integ, off); break;
-    case 2: k_kmul<D, 2><<<n, 256, 0, st>>>(rk, gk, c->utab, c->ctab, c->kd, c->cta_spec, blk0, c->d_sys, integ, off); break;
-    case 3: k_kmul<D, 3><<<n, 256, 0, st>>>(rk, gk, c->utab, c->ctab, c->kd, c->cta_spec, blk0, c->d_sys, integ, off); break;
-    case 4: k_kmul<D, 4><<<n, 256, 0, st>>>(rk, gk, c->utab, c->ctab, c->kd, c->cta_spec, blk0, c->d_sys, integ, off); break;
-    default: k_kmul<D, 0><<<n, 256, 0, st>>>(rk, gk, c->utab, c->ctab, c->kd, c->cta_spec, blk0, c->d_sys, integ, off); break;
+    case 1: k_kmul<D, 1><<<n, 256, 0, st>>>(rk, gk, c->utab, c->ctab, c->kd, c->cta_spec, blk0, c->d_sys, integ, c->ahead, off); break;
+    case 2: k_kmul<D, 2><<<n, 256, 0, st>>>(rk, gk, c->utab, c->ctab, c->kd, c->cta_spec, blk0, c->d_sys, integ, c->ahead, off); break;
+    case 3: k_kmul<D, 3><<<n, 256, 0, st>>>(rk, gk, c->utab, c->ctab, c->kd, c->cta_spec, blk0, c->d_sys, integ, c->ahead, off); break;
+    case 4: k_kmul<D, 4><<<n, 256, 0, st>>>(rk, gk, c->utab, c->ctab, c->kd, c->cta_spec, blk0, c->d_sys, integ, c->ahead, off); break;
+    default: k_kmul<D, 0><<<n, 256, 0, st>>>(rk, gk, c->utab, c->ctab, c->kd, c->cta_spec, blk0, c->d_sys, integ, c->ahead, off); break;
   }
 }
 
@@ -1580,8 +1581,8 @@ int tild_finish_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys, bo
   c->rho_ahead = tild_spreads_ahead(c, integrate);
   if (integrate) {
     tild_mark(c, STAGE_TAIL);
-    k_advance_steps<<<nblk(c->nsys, 128), 128, 0, c->stream>>>(c->d_sys, c->nsys);
-    c->launches++;
+    c->ahead++;
+    if (c->last_of_call && tild_advance_steps(c)) return TILD_ERR_CUDA;
     c->cur ^= 1;
     c->steps_since_sort++;
   }
@@ -1596,6 +1597,15 @@ int tild_finish_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys, bo
     h.have_forces = true;
   }
   return TILD_OK;
+}
+
+// Brings the device's step counters up to the steps that have been launched.
+int tild_advance_steps(tild_ctx* c) {
+  if (c->ahead == 0) return 0;
+  k_advance_steps<<<nblk(c->nsys, 128), 128, 0, c->stream>>>(c->d_sys, c->nsys, c->ahead);
+  c->launches++;
+  c->ahead = 0;
+  return tild_check(c, cudaGetLastError(), "advance");
 }
 
 // A system's densities as planar FP32 channels [(T + C)][M] into dst (device memory) on stream st:
