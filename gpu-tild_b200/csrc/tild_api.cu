@@ -353,6 +353,21 @@ int engine_create(const tild_config* cfgs, int nsys, int device, tild_ctx* c, co
   // order <= 1 spreads by global atomics, which the gather absorbs at no cost; the order >= 2
   // shared box costs the gather its L1 share and barriers (both measured on the B200)
   c->spread_ahead = cfgs[0].pmeorder <= 1 ? 1 : 0;
+  // Order >= 2 in 3D reads its 27 to 125 field nodes from 4x4x4 bricks: us a step linear / brick, 2.6M
+  // beads on 128^3 order 3 549 / 491, 45^3 order 2 56.5 / 55.8, 90^3 order 4 246 / 235.  Half the shared
+  // box where beads are dense enough that 256 of them stay within it (more CTAs per SM: the same blend
+  // 516 / 491, 45^3 57.6 / 55.8; at 0.45 beads per node and channel most chunks overflow it, 48^3 order 3
+  // 54.3 / 59.4).
+  if (cfgs[0].dim == 3 && cfgs[0].pmeorder >= 2) {
+    c->field_layout = TILD_FIELD_BRICK;
+    bool dense = cfgs[0].pmeorder <= 3;
+    for (int s = 0; s < nsys; s++) {
+      const tild_config& q = cfgs[s];
+      const double nodes = (double)q.nx[0] * q.nx[1] * q.nx[2] * (q.ntypes + (q.do_charges ? 1 : 0));
+      dense = dense && q.ns >= 0.55 * nodes;
+    }
+    if (dense) c->spread_cap = 6144;
+  }
   long long slots = 0, beads = 0, utab = 0, virk = 0, ctab = 0, kd = 0, fr = 0;
   // buckets by grid shape (order of first appearance)
   for (int s = 0; s < nsys; s++) {
