@@ -126,9 +126,12 @@ __device__ __forceinline__ void spread_global_kbits(const float (&W)[3][P + 1], 
 // The spread of one CTA's beads, positions already in registers (ok: this thread's bead is valid
 // and finite; t its type; q its charge, 0 without).  Thread 0's bead is the box origin.  Every
 // thread of the block must call it.  The spread kernel and the spreading gather share it.
-template <int D, int P, bool CH>
+//
+// TPB threads share a bead (all of a warp the same share): thread share `r` adds the (x, y) rows k of
+// the stencil with k mod TPB = r.
+template <int D, int P, bool CH, int TPB = 1>
 __device__ __forceinline__ void cta_spread_box(bool ok, const float (&xs)[3], int t, float q, const SysDev& sd,
-                                               unsigned long long* __restrict__ rho_fx, int cap, int* status) {
+                                               unsigned long long* __restrict__ rho_fx, int cap, int* status, int r = 0) {
   extern __shared__ __align__(16) int smi[];  // the box: cap words, cap a multiple of 4
   __shared__ int s_g0[3], s_min[3], s_max[3];
   __shared__ int s_row[kMaxRows];  // row offsets in one channel (grids hold fewer than 2^31 points)
@@ -176,6 +179,7 @@ __device__ __forceinline__ void cta_spread_box(bool ok, const float (&xs)[3], in
       for (int ix = 0; ix <= P; ix++)
 #pragma unroll
         for (int iy = 0; iy <= P; iy++) {
+          if (TPB > 1 && (ix * (P + 1) + iy) % TPB != r) continue;
           const int rowl = (rel[1] - mn[1] + iy) * ext[0] + (rel[0] - mn[0] + ix);
           const float wxy = W[0][ix] * W[1][iy] * sc32;
           if (D == 3) {
@@ -220,7 +224,7 @@ __device__ __forceinline__ void cta_spread_box(bool ok, const float (&xs)[3], in
         atomicAdd(gch + s_row[row] + xg, (unsigned long long)((long long)v << sh));
       }
     }
-  } else if (ok) {
+  } else if (ok && r == 0) {
     // the box does not fit: the same 2^kbits contributions, added to the global grid directly
     float W[3][P + 1];
 #pragma unroll
@@ -295,22 +299,27 @@ __device__ __forceinline__ bool spread_input(const float4& p, const SysDev& sd, 
 
 // 7 CTAs per SM (32 registers, a few spilled): the barriers of one CTA's box phases are covered
 // by the others (blend: 0.153 -> 0.144 ms against 48 registers and 5 CTAs)
-template <int D, int P, bool CH>
+//
+// TPB > 1: a CTA takes 256 / TPB slots of a 256-slot block, and each bead's stencil is shared by lanes of
+// TPB warps (spread_share says when).
+template <int D, int P, bool CH, int TPB>
 __global__ void __launch_bounds__(256, 7) k_spread_tiled(const float4* __restrict__ pos, const float* __restrict__ charge,
                                                      const int* __restrict__ cta_sys,
                                                      const SysDev* __restrict__ sysd,
                                                      unsigned long long* __restrict__ rho_fx_all, int cap,
                                                      int* status, int blk_off) {
-  const int blk = blockIdx.x + blk_off;
+  const int blk = blockIdx.x / TPB + blk_off;
   const SysDev& sd = sysd[cta_sys[blk]];  // inactive systems too (see k_fix_to_float)
   static_assert(kTile == 256, "the lane-to-slot map below assumes 8 warps of 32");
-  // lane l of warp w takes slot 8 l + w: a warp's beads lie in distinct cells, so its shared
-  // atomics meet fewer equal addresses; thread 0 keeps slot 0, the box origin
-  const int i = blk * blockDim.x + (((threadIdx.x & 31) << 3) | (threadIdx.x >> 5));
+  // lane l of warp w takes slot (8 / TPB) l + w mod (8 / TPB): a warp's beads lie in distinct cells, so its
+  // shared atomics meet fewer equal addresses; thread 0 keeps slot 0, the box origin
+  constexpr int W = 8 / TPB;
+  const int warp = threadIdx.x >> 5, r = warp / W;
+  const int i = blk * kTile + (blockIdx.x % TPB) * (kTile / TPB) + (threadIdx.x & 31) * W + warp % W;
   float xs[3], q;
   int t;
   const bool ok = spread_input<D, CH>(pos[i], sd, charge, i, xs, t, q, status);
-  cta_spread_box<D, P, CH>(ok, xs, t, q, sd, rho_fx_all + sd.grid0, cap, status);
+  cta_spread_box<D, P, CH, TPB>(ok, xs, t, q, sd, rho_fx_all + sd.grid0, cap, status, r);
 }
 
 // Every node straight into the 64-bit global accumulator: always for order <= 1, where a shared
@@ -1192,6 +1201,28 @@ struct BeadRange {
 };
 inline BeadRange all_beads(tild_ctx* c) { return {c->stream, 0, c->n_cta_bead}; }
 
+// Threads per bead of the box spread.  256 sorted beads cover about V = 256 / density nodes, a run of
+// V / 64 bricks along x; with the stencil's and two nodes of drift's halo their box has to fit the
+// largest shared box with room for a turn into the next row of bricks (40 %), or the chunk adds every
+// node to the global grid: 64^3, 4 channels, 0.49 beads per node, order 3: spread 98 us with 256 beads a
+// CTA, 36 with 64; 90^3 order 4, 0.41: 91 and 70.  Where they fit, fewer beads a CTA clear and flush more
+// words a bead (2.6M blend 126 and 337 us), except in systems that do not fill the SMs (10,000 beads:
+// 10.0 and 7.5 us; 60,000 of order 4: 26 and 20).
+int spread_share(const tild_ctx* c) {
+  if (c->n_cta_bead < 296) return 4;
+  int share = 1;
+  for (const SysHost& h : c->sys) {
+    const double density = (double)h.ns / (double)h.g.M;
+    const int edge = c->D == 3 ? 4 : 8, halo = c->P + 2;
+    auto words = [&](int beads) {
+      const double run = beads / density / 64.0 * edge + halo, side = edge + halo;
+      return 1.4 * (h.T + h.C) * run * side * (c->D == 3 ? side : 1.0);
+    };
+    while (share < 4 && words(256 / share) > 12288.0) share *= 2;
+  }
+  return share;
+}
+
 // CH: some system of the engine has charges (the kernels without it carry no charge code)
 template <int D, int P, bool CH>
 void launch_spread_k(tild_ctx* c, BeadRange r) {
@@ -1199,16 +1230,22 @@ void launch_spread_k(tild_ctx* c, BeadRange r) {
     k_spread_direct<D, P, CH><<<r.n, kTile, 0, r.st>>>(c->pos[c->cur], c->charge, c->cta_bead, c->d_sys, c->rho_fx,
                                                         c->d_status, r.off);
   } else if constexpr (P >= 2) {
-    static std::atomic<unsigned long long> attr_devices{0};  // one bit per device with the attribute set
-    const unsigned long long bit = 1ull << (c->device & 63);
-    if (!(attr_devices.load() & bit)) {
-      cudaFuncSetAttribute(k_spread_tiled<D, P, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)(sizeof(int) * 12288));
-      attr_devices.fetch_or(bit);
-    }
-    const size_t smem = sizeof(int) * (size_t)c->spread_cap;
-    k_spread_tiled<D, P, CH><<<r.n, kTile, smem, r.st>>>(c->pos[c->cur], c->charge, c->cta_bead, c->d_sys, c->rho_fx,
-                                                          c->spread_cap, c->d_status, r.off);
+    auto launch = [&](auto* kernel, int share) {
+      static std::atomic<unsigned long long> attr_devices{0};  // one bit per device with the attribute set
+      const unsigned long long bit = 1ull << (c->device & 63);
+      if (!(attr_devices.load() & bit)) {
+        for (auto* k : {k_spread_tiled<D, P, CH, 1>, k_spread_tiled<D, P, CH, 2>, k_spread_tiled<D, P, CH, 4>})
+          cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(int) * 12288));
+        attr_devices.fetch_or(bit);
+      }
+      const size_t smem = sizeof(int) * (size_t)c->spread_cap;
+      kernel<<<r.n * share, kTile, smem, r.st>>>(c->pos[c->cur], c->charge, c->cta_bead, c->d_sys, c->rho_fx, c->spread_cap,
+                                                 c->d_status, r.off);
+    };
+    const int share = spread_share(c);
+    if (share == 1) launch(k_spread_tiled<D, P, CH, 1>, 1);
+    else if (share == 2) launch(k_spread_tiled<D, P, CH, 2>, 2);
+    else launch(k_spread_tiled<D, P, CH, 4>, 4);
   }
 }
 

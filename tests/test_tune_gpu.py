@@ -142,3 +142,18 @@ def test_spread_ahead_after_host_changes(pmeorder):
     for a, b, r in zip(mid, again, ref):
         assert np.array_equal(a, b)
         assert np.array_equal(a, r)
+
+
+@pytest.mark.parametrize("edge,order", [(32, 3), (64, 4), (64, 3), (90, 2)])
+def test_box_spread_shares_give_the_direct_densities(edge, order):
+    """1, 2 or 4 threads per bead (chosen by density and size) add the contributions of the direct spread."""
+    s = small_diblock(3, order, nx=(edge,) * 3, box=(edge / 2.0,) * 3, n_chains=3801, N=20, seed=5)
+    rho = []
+    for mode in (tild.SPREAD_TILED, tild.SPREAD_DIRECT):
+        with tild.Context(s) as c:
+            t = c.get_tune()
+            t.spread_mode, t.spread_cap = mode, 12288
+            c.set_tune(t)
+            c.step(3)
+            rho.append(c.density())
+    assert np.array_equal(rho[0], rho[1])
