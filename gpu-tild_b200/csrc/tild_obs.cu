@@ -10,6 +10,7 @@
 //   E_el = sum_full 4 pi lB e^{-k^2/(2a^2)} / k^2 |rho_c(k)|^2 / M      (calc_properties.cu:106-116)
 // with sum_full = sum_half w(k) Re(...), w = 1 on the kx = 0 and Nyquist planes, else 2.
 #include "tild_internal.cuh"
+#include <algorithm>
 #include <cmath>
 
 namespace {
@@ -46,26 +47,75 @@ __device__ void block_sum_write(double (&v)[NV], double* out) {
   }
 }
 
-// one FFT pair style: energy and nP virial components
-__global__ void __launch_bounds__(kObsThreads) k_obs_style(const float2* __restrict__ rhok, const float* __restrict__ ut,
-                                                          const float2* __restrict__ vk, int a, int b, Geom g, int nP,
-                                                          double scale, double* __restrict__ partial) {
+// Every FFT pair style of a system in one launch: CTA (b, k) sums style k's energy and nP virial
+// components over its part of the half spectrum.  The loads of kObsBatch points are in flight per
+// thread (the kernels stream their tables once: nP complex and one float per point and style).
+struct ObsStyles {
+  int a[TILD_MAX_STYLES], b[TILD_MAX_STYLES];
+  double scale[TILD_MAX_STYLES];
+};
+constexpr int kObsBatch = 2;
+template <int NP>
+__global__ void __launch_bounds__(kObsThreads, 4) k_obs_styles(const float2* __restrict__ rhok, const float* __restrict__ ut_all,
+                                                           const float2* __restrict__ vk_all, const __grid_constant__ ObsStyles st,
+                                                           Geom g, double* __restrict__ partial) {
   double v[7] = {0, 0, 0, 0, 0, 0, 0};
+  const int k = blockIdx.y;
   const long long Mh = g.Mh;
-  for (long long h = blockIdx.x * (long long)blockDim.x + threadIdx.x; h < Mh; h += (long long)gridDim.x * blockDim.x) {
-    const int ix = (int)(h % g.nxh);
-    const double w = hermitian_weight(ix, g.nx[0]);
-    const float2 ra = rhok[(long long)a * Mh + h], rb = rhok[(long long)b * Mh + h];
-    // rho_b conj(rho_a)
-    const double re = (double)rb.x * ra.x + (double)rb.y * ra.y;
-    const double im = (double)rb.y * ra.x - (double)rb.x * ra.y;
-    v[0] += w * (double)ut[h] * scale * re;
-    for (int j = 0; j < nP; j++) {
-      const float2 q = vk[(long long)j * Mh + h];
-      v[1 + j] += w * ((double)q.x * re - (double)q.y * im);
+  const float2 *ra = rhok + st.a[k] * Mh, *rb = rhok + st.b[k] * Mh, *vk = vk_all + (long long)k * NP * Mh;
+  const float* ut = ut_all + k * Mh;
+  const double scale = st.scale[k];
+  const unsigned nxh = g.nxh, n = (unsigned)Mh, stride = gridDim.x * kObsThreads;
+  for (unsigned h0 = blockIdx.x * kObsThreads + threadIdx.x; h0 < n; h0 += kObsBatch * stride) {
+    float2 A[kObsBatch], B[kObsBatch], Q[kObsBatch][NP];
+    float U[kObsBatch];
+#pragma unroll
+    for (int q = 0; q < kObsBatch; q++) {
+      const unsigned h = h0 + q * stride;
+      const bool in = h < n;
+      A[q] = in ? ra[h] : make_float2(0.f, 0.f);
+      B[q] = in ? rb[h] : make_float2(0.f, 0.f);
+      U[q] = in ? ut[h] : 0.f;
+#pragma unroll
+      for (int j = 0; j < NP; j++) Q[q][j] = in ? vk[j * Mh + h] : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int q = 0; q < kObsBatch; q++) {
+      const unsigned h = h0 + q * stride;
+      const double w = hermitian_weight((int)(h % nxh), g.nx[0]);
+      // rho_b conj(rho_a)
+      const double re = w * ((double)B[q].x * A[q].x + (double)B[q].y * A[q].y);
+      const double im = w * ((double)B[q].y * A[q].x - (double)B[q].x * A[q].y);
+      v[0] += (double)U[q] * scale * re;
+#pragma unroll
+      for (int j = 0; j < NP; j++) v[1 + j] += (double)Q[q][j].x * re - (double)Q[q][j].y * im;
     }
   }
-  block_sum_write<7>(v, partial);
+  block_sum_write<7>(v, partial + 7ll * k * gridDim.x);
+}
+
+// Block g sums the partials of value g: groups of nv values in `blocks` partial rows each, in block order.
+struct ObsGroup {
+  int at, blocks, nv, first;  // first partial, rows, values per row, first result
+};
+struct ObsGroups {
+  ObsGroup g[TILD_MAX_STYLES + 2];
+  int n;
+};
+__global__ void __launch_bounds__(128) k_obs_sum(const double* __restrict__ partial, const __grid_constant__ ObsGroups groups,
+                                                 double* __restrict__ out) {
+  int k = 0;
+  while (k + 1 < groups.n && (int)blockIdx.x >= groups.g[k + 1].first) k++;
+  const ObsGroup g = groups.g[k];
+  const int j = blockIdx.x - g.first;
+  double s = 0.0;
+  for (int b = threadIdx.x; b < g.blocks; b += blockDim.x) s += partial[g.at + (long long)b * g.nv + j];
+  __shared__ double sh[4];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) out[blockIdx.x] = (sh[0] + sh[1]) + (sh[2] + sh[3]);
 }
 
 // smeared electrostatics: psi_k = 4 pi lB e^{-k^2/(2 a^2)} rho_c(k) / (M k^2), E = sum_r psi rho_c
@@ -75,10 +125,10 @@ __global__ void __launch_bounds__(kObsThreads) k_obs_charge(const float2* __rest
   double v[1] = {0.0};
   const long long Mh = g.Mh;
   for (long long h = blockIdx.x * (long long)blockDim.x + threadIdx.x; h < Mh; h += (long long)gridDim.x * blockDim.x) {
-    const int ix = (int)(h % g.nxh);
-    const long long r = h / g.nxh;
-    const int iy = (int)(r % g.nx[1]);
-    const int iz = (int)(r / g.nx[1]);
+    const unsigned r = (unsigned)h / (unsigned)g.nxh;  // grids hold fewer than 2^31 points
+    const int ix = (int)((unsigned)h - r * (unsigned)g.nxh);
+    const int iy = (int)(r % (unsigned)g.nx[1]);
+    const int iz = (int)(r / (unsigned)g.nx[1]);
     const int nn[3] = {ix, iy, iz};
     double k2 = 0.0;
     int off = 0;
@@ -332,18 +382,8 @@ int tild_ensure_red(tild_ctx* c, int nvals, int nblocks) {
   return TILD_OK;
 }
 
-static int reduce_host(tild_ctx* c, int nvals, int nblocks, double* out) {
-  std::vector<double> h((size_t)nvals * nblocks);
-  if (tild_check(c, cudaMemcpyAsync(h.data(), c->red, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->stream),
-                 "copy partials") ||
-      tild_check(c, cudaStreamSynchronize(c->stream), "sync partials"))
-    return TILD_ERR_CUDA;
-  for (int k = 0; k < nvals; k++) out[k] = 0.0;
-  for (int b = 0; b < nblocks; b++)
-    for (int k = 0; k < nvals; k++) out[k] += h[(size_t)b * nvals + k];
-  return TILD_OK;
-}
-
+// All terms of the observables are launched before anything is read back: one copy and one wait for
+// every style, the charges and the bonds (a wait per term was most of the 360 us of 6 styles on 96^3).
 int tild_obs_compute(tild_ctx* c, int si, tild_obs* o) {
   const SysHost& h = c->sys[si];
   const SysDev& hd = c->h_sys[si];
@@ -351,52 +391,79 @@ int tild_obs_compute(tild_ctx* c, int si, tild_obs* o) {
   o->n_styles = h.cfg.n_styles;
   o->n_p_comps = h.nP;
   o->step = h.forces_step;
-  const int nblocks = 296;
-  if (tild_ensure_red(c, 7, nblocks)) return TILD_ERR_OOM;
-  const float2* rk = tild_half_spectra(c, si);  // per-channel half spectra of the last force evaluation
-  if (!rk) return TILD_ERR_CUDA;
-  double upe = 0.0;
-  for (size_t k = 0; k < h.fft_cfg.size(); k++) {
-    const int ci = h.fft_cfg[k];
-    const double scale = ramp_ratio(hd, (int)k, h.forces_step);
-    k_obs_style<<<nblocks, kObsThreads, 0, c->stream>>>(rk, c->utab + h.utab0 + (long long)k * h.g.Mh,
-                                                         reinterpret_cast<const float2*>(c->virk) + h.virk0 +
-                                                             (long long)k * h.nP * h.g.Mh,
-                                                         hd.sa[k], hd.sb[k], h.g, h.nP, scale, c->red);
+  const int nfft = (int)h.fft_cfg.size();
+  const SysDev* dsys = c->d_sys + si;
+  // CTAs: enough to fill the SMs, no more than there are batches of points (or beads) for
+  auto ctas = [](long long items, long long most) { return (int)std::max(1ll, std::min(most, (items + kObsThreads - 1) / kObsThreads)); };
+  const int sblocks = ctas(h.g.Mh / kObsBatch, 1776 / std::max(nfft, 1));
+  const int bblocks = ctas(h.ns_pad, 1184), cblocks = h.C ? ctas(h.g.Mh, 1184) : 0;
+  ObsGroups gr;
+  gr.n = 0;
+  int at = 0, values = 0;
+  auto group = [&](int blocks, int nv) {
+    gr.g[gr.n++] = {at, blocks, nv, values};
+    at += blocks * nv;
+    values += nv;
+  };
+  for (int k = 0; k < nfft; k++) group(sblocks, 7);
+  const int bond0 = at;
+  group(bblocks, 7);
+  const int charge0 = at;
+  if (h.C) group(cblocks, 1);
+  if (tild_ensure_red(c, 1, at + values)) return TILD_ERR_OOM;
+  const float2* rk = nullptr;
+  if (nfft || h.C) {
+    rk = tild_half_spectra(c, si);  // per-channel half spectra of the last force evaluation
+    if (!rk) return TILD_ERR_CUDA;
+  }
+  if (nfft) {
+    ObsStyles st;
+    for (int k = 0; k < nfft; k++) {
+      st.a[k] = hd.sa[k];
+      st.b[k] = hd.sb[k];
+      st.scale[k] = ramp_ratio(hd, k, h.forces_step);
+    }
+    const float* ut = c->utab + h.utab0;
+    const float2* vk = reinterpret_cast<const float2*>(c->virk) + h.virk0;
+    const dim3 grid(sblocks, nfft);
+    if (h.nP == 6) k_obs_styles<6><<<grid, kObsThreads, 0, c->stream>>>(rk, ut, vk, st, h.g, c->red);
+    else k_obs_styles<3><<<grid, kObsThreads, 0, c->stream>>>(rk, ut, vk, st, h.g, c->red);
     c->launches++;
-    double r[7];
-    if (reduce_host(c, 7, nblocks, r)) return TILD_ERR_CUDA;
-    o->style_energy[ci] = r[0] * h.dV;
+  }
+  k_obs_bonds<<<bblocks, kObsThreads, 0, c->stream>>>(c->pos[c->cur], c->bead_id, c->bond_nbr, c->bond_info, dsys->bond_k,
+                                                       dsys->bond_req, h.g, h.D, h.slot0, h.ns_pad, c->red + bond0);
+  c->launches++;
+  if (h.C) {
+    k_obs_charge<<<cblocks, kObsThreads, 0, c->stream>>>(rk + (long long)h.T * h.g.Mh, c->kk + h.kd0, h.g, h.D,
+                                                          (double)h.cfg.bjerrum,
+                                                          (double)h.cfg.smearing * (double)h.cfg.smearing, c->red + charge0);
+    c->launches++;
+  }
+  k_obs_sum<<<values, 128, 0, c->stream>>>(c->red, gr, c->red + at);
+  c->launches++;
+  double v[7 * (TILD_MAX_STYLES + 1) + 1];
+  if (tild_check(c, cudaMemcpyAsync(v, c->red + at, sizeof(double) * values, cudaMemcpyDeviceToHost, c->stream), "copy sums") ||
+      tild_check(c, cudaStreamSynchronize(c->stream), "sync sums"))
+    return TILD_ERR_CUDA;
+  double upe = 0.0;
+  for (int k = 0; k < nfft; k++) {
+    const int ci = h.fft_cfg[k];
+    o->style_energy[ci] = v[7 * k] * h.dV;
     upe += o->style_energy[ci];
     for (int j = 0; j < h.nP; j++) {
-      o->style_virial[ci][j] = r[1 + j] * h.dV / h.V / (double)h.D;
+      o->style_virial[ci][j] = v[7 * k + 1 + j] * h.dV / h.V / (double)h.D;
       o->ptens[j] += o->style_virial[ci][j];
     }
   }
   if (h.C) {
-    k_obs_charge<<<nblocks, kObsThreads, 0, c->stream>>>(rk + (long long)h.T * h.g.Mh, c->kk + h.kd0, h.g, h.D,
-                                                          (double)h.cfg.bjerrum,
-                                                          (double)h.cfg.smearing * (double)h.cfg.smearing, c->red);
-    c->launches++;
-    double r[1];
-    if (reduce_host(c, 1, nblocks, r)) return TILD_ERR_CUDA;
-    o->uelec = r[0] / (double)h.g.M;
+    o->uelec = v[7 * nfft + 7] / (double)h.g.M;
     upe += o->uelec;
   }
-  {
-    const SysDev* dsys = c->d_sys + si;
-    k_obs_bonds<<<nblocks, kObsThreads, 0, c->stream>>>(c->pos[c->cur], c->bead_id, c->bond_nbr, c->bond_info,
-                                                         dsys->bond_k, dsys->bond_req, h.g, h.D, h.slot0, h.ns_pad,
-                                                         c->red);
-    c->launches++;
-    double r[7];
-    if (reduce_host(c, 7, nblocks, r)) return TILD_ERR_CUDA;
-    o->ubond = r[0];
-    upe += o->ubond;
-    for (int j = 0; j < h.nP; j++) {
-      o->bond_vir[j] = r[1 + j] * (1.0 / h.V / (double)h.D);
-      o->ptens[j] += o->bond_vir[j];
-    }
+  o->ubond = v[7 * nfft];
+  upe += o->ubond;
+  for (int j = 0; j < h.nP; j++) {
+    o->bond_vir[j] = v[7 * nfft + 1 + j] * (1.0 / h.V / (double)h.D);
+    o->ptens[j] += o->bond_vir[j];
   }
   o->upe = upe;
   return tild_check(c, cudaGetLastError(), "observables") ? TILD_ERR_CUDA : TILD_OK;
