@@ -281,6 +281,8 @@ struct tild_ctx {
   };
   std::vector<TablePlan> tab_plans;
   long long tab_M = 0;
+  bool tab_batch = false;                // a style's force tables and virial kernels are transformed together
+  double* tab_u0 = nullptr;              // u_s(0) of the system's styles
   double* tab_ufull = nullptr;
   cufftDoubleComplex* tab_z = nullptr;
   cufftDoubleComplex* tab_z2 = nullptr;

@@ -126,9 +126,11 @@ __global__ void k_charge_table(float* ctab, Geom g, int D, double lB, double a, 
 // F_beta(k) = -i kd_beta u(k) on the half spectrum, Nyquist derivative set to zero: its C2R
 // equals Re of the reference's full C2C inverse of f_k (the Nyquist plane of the derivative
 // direction only contributes imaginary values there).
-__global__ void k_force_kernel(cufftDoubleComplex* out, const double* ufull, Geom g, int D, int beta) {
+__global__ void k_force_kernel(cufftDoubleComplex* out, const double* ufull, Geom g, int D, int beta0) {
   const long long h = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (h >= g.Mh) return;
+  const int beta = beta0 + blockIdx.y;  // one direction per grid row
+  out += blockIdx.y * g.Mh;
   int n[3];
   half_index(h, g, n[0], n[1], n[2]);
   const int N = g.nx[beta];
@@ -140,9 +142,15 @@ __global__ void k_force_kernel(cufftDoubleComplex* out, const double* ufull, Geo
 
 // vr(r) = dr_alpha(r) * f_beta(r) with dr the minimum image of the grid point from the origin
 // evaluated in FP32 as d_initVirial does (device_array_utils.cu:456-494).
-__global__ void k_virial_real(double* vr, const double* fbeta, Geom g, int D, int alpha) {
+// One component j0 + blockIdx.y per grid row; the force tables and the products lie Mpad apart.
+__global__ void k_virial_real(double* vr, const double* freal, Geom g, int D, long long Mpad, int j0) {
   const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (id >= g.M) return;
+  const int j = j0 + blockIdx.y;
+  // (alpha, beta) of xx yy zz xy xz yz (3D), xx yy xy (2D)
+  const int alpha = j < D ? j : (D == 3 ? (j == 3 ? 1 : 2) : 1), beta = j < D ? j : (j == 5 ? 1 : 0);
+  const double* fbeta = freal + beta * Mpad;
+  vr += blockIdx.y * Mpad;
   int nn[3] = {0, 0, 0};
   long long r = id;
   nn[0] = (int)(r % g.nx[0]);
@@ -159,6 +167,8 @@ __global__ void k_virial_real(double* vr, const double* fbeta, Geom g, int D, in
 __global__ void k_store_virk(cufftComplex* dst, const cufftDoubleComplex* src, long long Mh, double scale) {
   const long long h = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (h >= Mh) return;
+  dst += blockIdx.y * Mh;
+  src += blockIdx.y * Mh;
   dst[h].x = (float)(src[h].x * scale);
   dst[h].y = (float)(src[h].y * scale);
 }
@@ -229,7 +239,6 @@ int tild_build_tables(tild_ctx* c, int si) {
     }
     if (tild_check(c, cudaMemcpyAsync(c->kk + h.kd0, kk.data(), kk.size() * 4, cudaMemcpyHostToDevice, st), "copy k")) return TILD_ERR_CUDA;
     if (tild_check(c, cudaMemcpyAsync(c->kd + h.kd0, kd.data(), kd.size() * 4, cudaMemcpyHostToDevice, st), "copy kd")) return TILD_ERR_CUDA;
-    if (tild_check(c, cudaStreamSynchronize(st), "sync k")) return TILD_ERR_CUDA;
   }
 
   const int nfft = (int)h.fft_cfg.size();
@@ -249,6 +258,10 @@ int tild_build_tables(tild_ctx* c, int si) {
   double* freal = c->tab_freal;
   double* vr = c->tab_vr;
   SysDev& hd = c->h_sys[si];
+  // the D force tables and nP virial kernels of a style go through the transforms together (one by one
+  // their launches were most of the 685 us of loading a slot)
+  const int nf = c->tab_batch ? D : 1, nv = c->tab_batch ? h.nP : 1;
+  double u0[TILD_MAX_STYLES];
   for (int s = 0; s < nfft && rc == TILD_OK; s++) {
     const tild_pair_style& ps = h.cfg.styles[h.fft_cfg[s]];
     StyleParams sp;
@@ -261,31 +274,27 @@ int tild_build_tables(tild_ctx* c, int si) {
     sp.Rf = ps.rp;
     k_style_table<<<nblk(g.Mh, 256), 256, 0, st>>>(c->utab + h.utab0 + (long long)s * g.Mh, ufull, sp, g, D, ref, invM);
     c->launches++;
-    double u0 = 0.0;
-    if (tild_check(c, cudaMemcpyAsync(&u0, ufull, sizeof(double), cudaMemcpyDeviceToHost, st), "u0") ||
-        tild_check(c, cudaStreamSynchronize(st), "sync u0")) { rc = TILD_ERR_CUDA; break; }
-    hd.suk0[s] = (float)u0;
-    // real-space force table f_beta(r), unnormalised inverse transform
-    for (int beta = 0; beta < D && rc == TILD_OK; beta++) {
-      k_force_kernel<<<nblk(g.Mh, 256), 256, 0, st>>>(zbuf, ufull, g, D, beta);
+    if (tild_check(c, cudaMemcpyAsync(c->tab_u0 + s, ufull, sizeof(double), cudaMemcpyDeviceToDevice, st), "u0")) { rc = TILD_ERR_CUDA; break; }
+    // real-space force tables f_beta(r), unnormalised inverse transforms
+    for (int beta = 0; beta < D && rc == TILD_OK; beta += nf) {
+      k_force_kernel<<<dim3(nblk(g.Mh, 256), nf), 256, 0, st>>>(zbuf, ufull, g, D, beta);
       c->launches++;
       if (tild_check_fft(c, cufftExecZ2D(pz2d, zbuf, freal + (long long)beta * Mpad), "exec z2d")) rc = TILD_ERR_CUDA;
     }
     // virial kernels: FFT(dr_alpha f_beta) / M (InitializeVirial), times the 1/M that
     // CalcVirial applies to rho_k (pair_style.cu:277-279), stored on the half spectrum.
-    const int ab[6][2] = {{0, 0}, {1, 1}, {2, 2}, {1, 0}, {2, 0}, {2, 1}};   // (alpha, beta)
-    const int ab2[3][2] = {{0, 0}, {1, 1}, {1, 0}};
-    for (int j = 0; j < h.nP && rc == TILD_OK; j++) {
-      const int alpha = (D == 3) ? ab[j][0] : ab2[j][0];
-      const int beta = (D == 3) ? ab[j][1] : ab2[j][1];
-      k_virial_real<<<nblk(g.M, 256), 256, 0, st>>>(vr, freal + (long long)beta * Mpad, g, D, alpha);
+    for (int j = 0; j < h.nP && rc == TILD_OK; j += nv) {
+      k_virial_real<<<dim3(nblk(g.M, 256), nv), 256, 0, st>>>(vr, freal, g, D, Mpad, j);
       c->launches++;
       if (tild_check_fft(c, cufftExecD2Z(pd2z, vr, zbuf2), "exec d2z")) { rc = TILD_ERR_CUDA; break; }
-      k_store_virk<<<nblk(g.Mh, 256), 256, 0, st>>>(c->virk + h.virk0 + ((long long)s * h.nP + j) * g.Mh, zbuf2, g.Mh,
-                                                    invM * invM);
+      k_store_virk<<<dim3(nblk(g.Mh, 256), nv), 256, 0, st>>>(c->virk + h.virk0 + ((long long)s * h.nP + j) * g.Mh, zbuf2, g.Mh,
+                                                              invM * invM);
       c->launches++;
     }
   }
+  if (rc == TILD_OK && nfft > 0 &&
+      tild_check(c, cudaMemcpyAsync(u0, c->tab_u0, sizeof(double) * nfft, cudaMemcpyDeviceToHost, st), "u0"))
+    rc = TILD_ERR_CUDA;
   if (rc == TILD_OK && h.C) {
     k_charge_table<<<nblk(g.Mh, 256), 256, 0, st>>>(c->ctab + h.ctab0, g, D, h.cfg.bjerrum, h.cfg.smearing, ref, invM);
     c->launches++;
@@ -299,6 +308,7 @@ int tild_build_tables(tild_ctx* c, int si) {
     c->launches++;
   }
   if (rc == TILD_OK && tild_check(c, cudaStreamSynchronize(st), "table build")) rc = TILD_ERR_CUDA;
+  for (int s = 0; s < nfft && rc == TILD_OK; s++) hd.suk0[s] = (float)u0[s];
   return rc;
 }
 
@@ -314,11 +324,15 @@ int tild_table_scratch(tild_ctx* c) {
     D = h.D;
   }
   const long long Mpad = (M + 1) / 2 * 2;
+  // whole styles at a time up to 2^21 points (0.4 GB of scratch at 128^3), above that one table
+  c->tab_batch = M <= (1ll << 21);
+  const int nf = c->tab_batch ? D : 1, nv = c->tab_batch ? (D == 3 ? 6 : 3) : 1;
   if (tild_check(c, cudaMalloc(&c->tab_ufull, sizeof(double) * Mh), "alloc table scratch") ||
-      tild_check(c, cudaMalloc(&c->tab_z, sizeof(cufftDoubleComplex) * Mh), "alloc table scratch") ||
-      tild_check(c, cudaMalloc(&c->tab_z2, sizeof(cufftDoubleComplex) * Mh), "alloc table scratch") ||
+      tild_check(c, cudaMalloc(&c->tab_u0, sizeof(double) * TILD_MAX_STYLES), "alloc table scratch") ||
+      tild_check(c, cudaMalloc(&c->tab_z, sizeof(cufftDoubleComplex) * Mh * nf), "alloc table scratch") ||
+      tild_check(c, cudaMalloc(&c->tab_z2, sizeof(cufftDoubleComplex) * Mh * nv), "alloc table scratch") ||
       tild_check(c, cudaMalloc(&c->tab_freal, sizeof(double) * Mpad * D), "alloc table scratch") ||
-      tild_check(c, cudaMalloc(&c->tab_vr, sizeof(double) * M), "alloc table scratch"))
+      tild_check(c, cudaMalloc(&c->tab_vr, sizeof(double) * Mpad * nv), "alloc table scratch"))
     return TILD_ERR_OOM;
   c->tab_M = M;
   return TILD_OK;
@@ -338,9 +352,15 @@ int tild_table_plans(tild_ctx* c, const Geom& g, int D, cufftHandle* z2d, cufftH
   tild_ctx::TablePlan tp;
   for (int q = 0; q < 3; q++) tp.nx[q] = g.nx[q];
   tp.z2d = tp.d2z = 0;
-  if (tild_check_fft(c, cufftPlanMany(&tp.z2d, D, n, nullptr, 1, 0, nullptr, 1, 0, CUFFT_Z2D, 1), "plan z2d"))
+  // complex lines Mh apart, real ones on 16-byte boundaries
+  const int nf = c->tab_batch ? D : 1, nv = c->tab_batch ? (D == 3 ? 6 : 3) : 1;
+  const int Mpad = (int)((g.M + 1) / 2 * 2), Mh = (int)g.Mh;
+  int real[3], half[3];
+  for (int q = 0; q < D; q++) real[q] = half[q] = n[q];
+  half[D - 1] = g.nxh;
+  if (tild_check_fft(c, cufftPlanMany(&tp.z2d, D, n, half, 1, Mh, real, 1, Mpad, CUFFT_Z2D, nf), "plan z2d"))
     return TILD_ERR_CUDA;
-  if (tild_check_fft(c, cufftPlanMany(&tp.d2z, D, n, nullptr, 1, 0, nullptr, 1, 0, CUFFT_D2Z, 1), "plan d2z")) {
+  if (tild_check_fft(c, cufftPlanMany(&tp.d2z, D, n, real, 1, Mpad, half, 1, Mh, CUFFT_D2Z, nv), "plan d2z")) {
     cufftDestroy(tp.z2d);
     return TILD_ERR_CUDA;
   }
@@ -362,10 +382,10 @@ void tild_tables_free(tild_ctx* c) {
     cufftDestroy(tp.d2z);
   }
   c->tab_plans.clear();
-  void* ptrs[] = {c->tab_ufull, c->tab_z, c->tab_z2, c->tab_freal, c->tab_vr};
+  void* ptrs[] = {c->tab_ufull, c->tab_u0, c->tab_z, c->tab_z2, c->tab_freal, c->tab_vr};
   for (void* p : ptrs)
     if (p) cudaFree(p);
-  c->tab_ufull = nullptr;
+  c->tab_ufull = c->tab_u0 = nullptr;
   c->tab_z = c->tab_z2 = nullptr;
   c->tab_freal = c->tab_vr = nullptr;
 }
