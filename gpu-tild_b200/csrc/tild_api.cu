@@ -257,6 +257,7 @@ void set_geometry(SysHost& h, const tild_config& cfg) {
     g.L[d] = (d < h.D) ? cfg.box[d] : 1.0f;
     g.Lh[d] = 0.5f * g.L[d];
     g.dx[d] = g.L[d] / (float)g.nx[d];
+    g.rdx[d] = 1.0f / g.dx[d];
   }
   h.dV = 1.0;
   h.V = 1.0;
@@ -314,6 +315,15 @@ void set_params(tild_ctx* c, int s) {
     d.type_mask[t] = h.type_integ_mask[t];
     d.mass[t] = cfg.mass[t];
     d.diff[t] = cfg.diff[t];
+    // device_GJF_integrator.cu:25-40, in its FP32 operations
+    const float m = cfg.mass[t], df = cfg.diff[t], delt = cfg.delt;
+    const float b = m / (m + delt / (2.0f * df));
+    const float delt2 = delt * delt;
+    d.gjf_2b[t] = 2.0f * b;
+    d.gjf_a[t] = (1.0f - delt / (2.0f * df * m)) / (1.0f + delt / (2.0f * df * m));
+    d.gjf_f[t] = b * delt2 / m;
+    d.gjf_n[t] = b * delt / (2.0f * m);
+    d.gjf_amp[t] = cfg.noise_mag / df;
   }
   for (int b = 0; b < cfg.n_bond_types; b++) {
     d.bond_k[b] = cfg.bond_k[b];

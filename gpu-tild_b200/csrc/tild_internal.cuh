@@ -46,6 +46,7 @@ struct Geom {
   int nx[3];
   int nxh;          // Nx/2 + 1
   float dx[3];      // L / Nx in FP32 (initialize.cu:36)
+  float rdx[3];     // 1 / dx, correctly rounded (div_by)
   float L[3];
   float Lh[3];      // 0.5f * L (config_utils.cu:46)
   float gvol;       // product of dx
@@ -85,6 +86,8 @@ struct SysDev {
   int integ_kind[TILD_MAX_INTEGRATORS];
   int type_mask[TILD_MAX_TYPES];
   float mass[TILD_MAX_TYPES], diff[TILD_MAX_TYPES];
+  // GJF of each type: 2b, a, b dt^2 / m, b dt / 2m and the noise amplitude (set_params)
+  float gjf_2b[TILD_MAX_TYPES], gjf_a[TILD_MAX_TYPES], gjf_f[TILD_MAX_TYPES], gjf_n[TILD_MAX_TYPES], gjf_amp[TILD_MAX_TYPES];
   float bond_k[TILD_MAX_BOND_TYPES], bond_req[TILD_MAX_BOND_TYPES];
 };
 
@@ -389,11 +392,22 @@ __device__ __forceinline__ float2 pair_unpack(float2 z, float2 zm, int second) {
                 : make_float2(0.5f * (z.x + zm.x), 0.5f * (z.y - zm.y));
 }
 
+// x / d correctly rounded, given r = 1 / d correctly rounded: two residual corrections of x r, the last
+// of a quotient that is already within an ulp, which Markstein's theorem makes exact (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000", 1990).  A bead takes 6 such
+// divisions for its stencil at order 1 and 18 at order 3, twice with its spread; five operations each
+// instead of a call with a range check.
+__device__ __forceinline__ float div_by(float x, float d, float r) {
+  float q = __fmul_rn(x, r);
+  q = __fmaf_rn(__fmaf_rn(-q, d, x), r, q);
+  return __fmaf_rn(__fmaf_rn(-q, d, x), r, q);
+}
+
 // spline_get_weights (device_grid_utils.cu:3-49), FP32, including the order-4 quirk
 // sx3 = sx2*sx2 of line 39.
 template <int P>
-__device__ __forceinline__ void spline_w(float gdx, float H, float* W) {
-  const float sx = gdx / H;
+__device__ __forceinline__ void spline_w(float gdx, float H, float rH, float* W) {
+  const float sx = div_by(gdx, H, rH);
   if (P == 0) {
     W[0] = 1.f;
   } else if (P == 1) {
@@ -406,17 +420,17 @@ __device__ __forceinline__ void spline_w(float gdx, float H, float* W) {
     W[2] = 0.125f + 0.5f * sx + 0.5f * sx2;
   } else if (P == 3) {
     const float sx2 = sx * sx, sx3 = sx2 * sx;
-    W[0] = (1.f - 6.f * sx + 12.f * sx2 - 8.f * sx3) / 48.f;
-    W[1] = (23.f - 30.f * sx - 12.f * sx2 + 24.f * sx3) / 48.f;
-    W[2] = (23.f + 30.f * sx - 12.f * sx2 - 24.f * sx3) / 48.f;
-    W[3] = (1.f + 6.f * sx + 12.f * sx2 + 8.f * sx3) / 48.f;
+    W[0] = div_by((1.f - 6.f * sx + 12.f * sx2 - 8.f * sx3), 48.f, 1.f / 48.f);
+    W[1] = div_by((23.f - 30.f * sx - 12.f * sx2 + 24.f * sx3), 48.f, 1.f / 48.f);
+    W[2] = div_by((23.f + 30.f * sx - 12.f * sx2 - 24.f * sx3), 48.f, 1.f / 48.f);
+    W[3] = div_by((1.f + 6.f * sx + 12.f * sx2 + 8.f * sx3), 48.f, 1.f / 48.f);
   } else {
     const float sx2 = sx * sx, sx3 = sx2 * sx2, sx4 = sx2 * sx2;
-    W[0] = (1.f - 8.f * sx + 24.f * sx2 - 32.f * sx3 + 16.f * sx4) / 384.f;
-    W[1] = (19.f - 44.f * sx + 24.f * sx2 + 16.f * sx3 - 16.f * sx4) / 96.f;
-    W[2] = (115.f - 120.f * sx2 + 48.f * sx4) / 192.f;
-    W[3] = (19.f + 44.f * sx + 24.f * sx2 - 16.f * sx3 - 16.f * sx4) / 96.f;
-    W[4] = (1.f + 8.f * sx + 24.f * sx2 + 32.f * sx3 + 16.f * sx4) / 384.f;
+    W[0] = div_by((1.f - 8.f * sx + 24.f * sx2 - 32.f * sx3 + 16.f * sx4), 384.f, 1.f / 384.f);
+    W[1] = div_by((19.f - 44.f * sx + 24.f * sx2 + 16.f * sx3 - 16.f * sx4), 96.f, 1.f / 96.f);
+    W[2] = div_by((115.f - 120.f * sx2 + 48.f * sx4), 192.f, 1.f / 192.f);
+    W[3] = div_by((19.f + 44.f * sx + 24.f * sx2 - 16.f * sx3 - 16.f * sx4), 96.f, 1.f / 96.f);
+    W[4] = div_by((1.f + 8.f * sx + 24.f * sx2 + 32.f * sx3 + 16.f * sx4), 384.f, 1.f / 384.f);
   }
 }
 
@@ -424,13 +438,13 @@ __device__ __forceinline__ void spline_w(float gdx, float H, float* W) {
 // nearest node, odd orders the containing cell; returns the first stencil node and sets gdx, the
 // offset from that node or cell centre that the spline weights take.
 template <int P>
-__device__ __forceinline__ int axis_index(float xj, float dxj, float& gdx) {
+__device__ __forceinline__ int axis_index(float xj, float dxj, float rdx, float& gdx) {
   int gi;
   if (P % 2 == 0) {
-    gi = (int)((xj + 0.5f * dxj) / dxj);
+    gi = (int)div_by(xj + 0.5f * dxj, dxj, rdx);
     gdx = xj - (float)gi * dxj;
   } else {
-    gi = (int)(xj / dxj);
+    gi = (int)div_by(xj, dxj, rdx);
     gdx = xj - ((float)gi + 0.5f) * dxj;
   }
   return gi - P / 2;
@@ -438,10 +452,10 @@ __device__ __forceinline__ int axis_index(float xj, float dxj, float& gdx) {
 
 // Grid index and weights of one bead along one axis.
 template <int P>
-__device__ __forceinline__ int axis_base(float xj, float dxj, float* W) {
+__device__ __forceinline__ int axis_base(float xj, float dxj, float rdx, float* W) {
   float gdx;
-  const int b = axis_index<P>(xj, dxj, gdx);
-  spline_w<P>(gdx, dxj, W);
+  const int b = axis_index<P>(xj, dxj, rdx, gdx);
+  spline_w<P>(gdx, dxj, rdx, W);
   return b;
 }
 

@@ -217,7 +217,7 @@ __global__ void k_stencil(const float4* __restrict__ pos, const int* __restrict_
   float W[3][P + 1];
   int idx[3][P + 1];
   for (int d = 0; d < D; d++) {
-    const int b = axis_base<P>(xs[d], g.dx[d], W[d]);
+    const int b = axis_base<P>(xs[d], g.dx[d], g.rdx[d], W[d]);
     for (int a = 0; a <= P; a++) idx[d][a] = wrap_idx(b + a, g.nx[d], status);
   }
   constexpr int S = (D == 3) ? (P + 1) * (P + 1) * (P + 1) : (P + 1) * (P + 1);

@@ -78,7 +78,7 @@ __device__ __forceinline__ void chunk_origin(const float4* __restrict__ pos, int
     float Wd[P + 1];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-      s_g0[d] = (valid && d < D && isfinite(x0[d])) ? axis_base<P>(x0[d], g.dx[d], Wd) : 0;
+      s_g0[d] = (valid && d < D && isfinite(x0[d])) ? axis_base<P>(x0[d], g.dx[d], g.rdx[d], Wd) : 0;
       s_min[d] = INT_MAX;
       s_max[d] = INT_MIN;
     }
@@ -141,7 +141,7 @@ __device__ __forceinline__ void cta_spread_box(bool ok, const float (&xs)[3], in
     float Wd[P + 1];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-      s_g0[d] = (ok && d < D) ? axis_base<P>(xs[d], g.dx[d], Wd) : 0;
+      s_g0[d] = (ok && d < D) ? axis_base<P>(xs[d], g.dx[d], g.rdx[d], Wd) : 0;
       s_min[d] = INT_MAX;
       s_max[d] = INT_MIN;
     }
@@ -152,7 +152,7 @@ __device__ __forceinline__ void cta_spread_box(bool ok, const float (&xs)[3], in
   int rel[3] = {0, 0, 0};
   if (ok) {
 #pragma unroll
-    for (int d = 0; d < D; d++) rel[d] = fold_rel(axis_index<P>(xs[d], g.dx[d], gd[d]) - s_g0[d], g.nx[d]);
+    for (int d = 0; d < D; d++) rel[d] = fold_rel(axis_index<P>(xs[d], g.dx[d], g.rdx[d], gd[d]) - s_g0[d], g.nx[d]);
   }
   int mn[3], ext[3];
   long long vol;
@@ -171,7 +171,7 @@ __device__ __forceinline__ void cta_spread_box(bool ok, const float (&xs)[3], in
     if (ok) {
       float W[3][P + 1];
 #pragma unroll
-      for (int d = 0; d < D; d++) spline_w<P>(gd[d], g.dx[d], W[d]);
+      for (int d = 0; d < D; d++) spline_w<P>(gd[d], g.dx[d], g.rdx[d], W[d]);
       const float sc32 = ig * __int_as_float((127 + kbits) << 23);  // 2^kbits / gvol
       int* st = smi + (long long)t * vol;
       int* sq = smi + (long long)T * vol;
@@ -228,7 +228,7 @@ __device__ __forceinline__ void cta_spread_box(bool ok, const float (&xs)[3], in
     // the box does not fit: the same 2^kbits contributions, added to the global grid directly
     float W[3][P + 1];
 #pragma unroll
-    for (int d = 0; d < D; d++) spline_w<P>(gd[d], g.dx[d], W[d]);
+    for (int d = 0; d < D; d++) spline_w<P>(gd[d], g.dx[d], g.rdx[d], W[d]);
     int idx[3][P + 1];
 #pragma unroll
     for (int d = 0; d < D; d++)
@@ -252,7 +252,7 @@ __device__ __forceinline__ void bead_spread_direct(const float (&xs)[3], int t, 
   int idx[3][P + 1];
 #pragma unroll
   for (int d = 0; d < D; d++) {
-    const int b = axis_base<P>(xs[d], g.dx[d], W[d]);
+    const int b = axis_base<P>(xs[d], g.dx[d], g.rdx[d], W[d]);
 #pragma unroll
     for (int a = 0; a <= P; a++) idx[d][a] = pmod(b + a, g.nx[d]);
   }
@@ -845,17 +845,15 @@ __device__ __forceinline__ void bead_epilogue(int i, const float4& p, int t, flo
         for (int d = 0; d < D; d++) on[d] = noise[3 * (long long)i + d];
         any_gjf = true;
       }
-      const float m = sd.mass[t], df = sd.diff[t], delt = sd.delt;
-      const float b = m / (m + delt / (2.0f * df));
-      const float a = (1.0f - delt / (2.0f * df * m)) / (1.0f + delt / (2.0f * df * m));
-      const float delt2 = delt * delt;
+      // the type's constants come from the host, in the same FP32 operations: nine divisions a bead less
+      const float b2 = sd.gjf_2b[t], a = sd.gjf_a[t], cf = sd.gjf_f[t], cn = sd.gjf_n[t], amp = sd.gjf_amp[t];
 #pragma unroll
       for (int d = 0; d < D; d++) {
-        const float nn = sd.noise_mag / df * z[d];
+        const float nn = amp * z[d];
         const float xtmp = x[d];
         if (xo[d] - x[d] > g.L[d] / 2.0f) xo[d] -= g.L[d];
         else if (xo[d] - x[d] < -g.L[d] / 2.0f) xo[d] += g.L[d];
-        float xn = 2.0f * b * x[d] - a * xo[d] + b * delt2 / m * f[d] + b * delt / (2.0f * m) * (nn + on[d]);
+        float xn = b2 * x[d] - a * xo[d] + cf * f[d] + cn * (nn + on[d]);
         xo[d] = xtmp;
         on[d] = nn;
         if (xn > g.L[d]) xn -= g.L[d];
@@ -918,7 +916,7 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : (P >= 3 ? 4 : (P >= 2 ? 3 :
       int idx[3][4];
 #pragma unroll
       for (int d = 0; d < 3; d++) {
-        const int b = axis_base<3>(x[d], g.dx[d], W[d]);
+        const int b = axis_base<3>(x[d], g.dx[d], g.rdx[d], W[d]);
 #pragma unroll
         for (int a = 0; a <= 3; a++) idx[d][a] = wrap_idx(b + a, g.nx[d], status);
       }
@@ -960,7 +958,7 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : (P >= 3 ? 4 : (P >= 2 ? 3 :
       int idx[3][P + 1];
 #pragma unroll
       for (int d = 0; d < D; d++) {
-        const int b = axis_base<P>(x[d], g.dx[d], W[d]);
+        const int b = axis_base<P>(x[d], g.dx[d], g.rdx[d], W[d]);
 #pragma unroll
         for (int a = 0; a <= P; a++) idx[d][a] = wrap_idx(b + a, g.nx[d], status);
       }
@@ -1062,7 +1060,7 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : 3)) k_gather_box(
   if (ok) {
 #pragma unroll
     for (int d = 0; d < D; d++) {
-      base[d] = axis_base<P>(x[d], g.dx[d], W[d]);
+      base[d] = axis_base<P>(x[d], g.dx[d], g.rdx[d], W[d]);
       if (base[d] < -g.nx[d] || base[d] + P >= 2 * g.nx[d]) atomicOr(status, ST_INDEX_RANGE);
       rel[d] = fold_rel(base[d] - s_g0[d], g.nx[d]);
     }

@@ -87,3 +87,36 @@ def test_densities_belong_to_the_last_step_of_a_call():
         assert np.array_equal(a.density(), b.density())
         oa, ob = a.observables(), b.observables()
         assert oa["upe"] == ob["upe"] and np.array_equal(oa["ptens"], ob["ptens"])
+
+
+@pytest.mark.parametrize("order", [0, 1])
+def test_stencil_divisions_are_correctly_rounded(order):
+    """Indices and weights with node spacings that are no binary fractions: the FP32 division results."""
+    nx, box = (23, 37, 41), (7.3, 11.1, 13.7)
+    s = _system(nx)
+    rng = np.random.default_rng(8)
+    L = np.array(box, np.float32)
+    dx = L / np.array(nx, np.float32)
+    x = (rng.random((20000, 3)) * L).astype(np.float32)
+    x[:3000] = (rng.integers(0, 23, (3000, 3)) * dx).astype(np.float32)   # on or next to node planes
+    x = np.minimum(x, L)
+    n = len(x)
+    z = np.zeros((n, 3), np.int32)
+    s = tild.System(dim=3, nx=nx, box=box, types=np.zeros(n, np.int32), x=x, n_bonds=np.zeros(n, np.int32), bonded_to=z,
+                    bond_type=z, ntypes=1, styles=[Style(tild.STYLE_GAUSSIAN, 0, 0, 1.0, 0.7)], pmeorder=order)
+    with tild.Context(s) as c:
+        inds, w = c.stencil()
+    gi = ((x + np.float32(0.5) * dx) / dx if order == 0 else x / dx).astype(np.int64)
+    if order == 0:
+        W = [[np.ones(n, np.float32)] for _ in range(3)]
+    else:  # x - (gi + 0.5) dx is one fused operation on the device: exact in double, then rounded
+        gdx = (x.astype(np.float64) - (gi + 0.5) * dx.astype(np.float64)).astype(np.float32)
+        sx = gdx / dx
+        W = [[np.float32(0.5) - sx[:, d], np.float32(0.5) + sx[:, d]] for d in range(3)]
+    gvol = np.float32(dx[0] * dx[1]) * dx[2]
+    k = 0
+    for a in np.ndindex(*([order + 1] * 3)):
+        i = [(gi[:, d] + a[d]) % nx[d] for d in range(3)]
+        assert np.array_equal(inds[:, k], i[0] + (i[1] + i[2] * nx[1]) * nx[0])
+        assert np.array_equal(w[:, k], W[0][a[0]] * W[1][a[1]] * W[2][a[2]] / gvol)
+        k += 1
