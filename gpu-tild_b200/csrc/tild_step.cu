@@ -788,13 +788,16 @@ __device__ __forceinline__ void field_offsets(const int (&idx)[3][P + 1], int la
 
 // Bonds, the force output and the integrators of one bead: d_bonds (device_bonds.cu:4-60) and
 // Integrate_2 (integrator.cu:24-39) over the integrators in input order.  Shared by both gathers.
-template <int D, bool INTEG, bool XW>
+// PRE: the bead's previous noise (on0) and the normals of its first integrator (z0, of integrator ig0)
+// were fetched and drawn before.
+template <int D, bool INTEG, bool XW, bool PRE = false>
 __device__ __forceinline__ void bead_epilogue(int i, const float4& p, int t, float (&x)[3], float (&f)[3],
                                               const SysDev& sd, const Geom& g, int info, int nb,
                                               const float4 (&pj)[3], int bid, const float4& po,
                                               float* __restrict__ noise, float4* __restrict__ pos_io,
                                               float* __restrict__ f_out, int f_sys, int s,
-                                              curandStateXORWOW_t* __restrict__ xw, int ahead) {
+                                              curandStateXORWOW_t* __restrict__ xw, int ahead, const float* on0 = nullptr,
+                                              const float* z0 = nullptr, int ig0 = -1) {
   // bonds
 #pragma unroll
   for (int bb = 0; bb < 3; bb++) {
@@ -836,13 +839,16 @@ __device__ __forceinline__ void bead_epilogue(int i, const float4& p, int t, flo
     if (XW) {
 #pragma unroll
       for (int d = 0; d < D; d++) z[d] = curand_normal(&st);
+    } else if (PRE && ig == ig0) {
+#pragma unroll
+      for (int d = 0; d < D; d++) z[d] = z0[d];
     } else {
       philox_normal3(sd.seed, (uint32_t)bid, est, (uint32_t)ig, z);
     }
     if (sd.integ_kind[ig] == TILD_INTEGRATOR_GJF) {
       if (!any_gjf) {
 #pragma unroll
-        for (int d = 0; d < D; d++) on[d] = noise[3 * (long long)i + d];
+        for (int d = 0; d < D; d++) on[d] = PRE ? on0[d] : noise[3 * (long long)i + d];
         any_gjf = true;
       }
       // the type's constants come from the host, in the same FP32 operations: nine divisions a bead less
@@ -882,14 +888,22 @@ __device__ __forceinline__ void bead_epilogue(int i, const float4& p, int t, flo
 // accumulator for the next step, through the shared box (1) or the global atomics (2), so the
 // next step needs no spread kernel.  Inactive systems spread their held positions.  The integer
 // sums are those of the spread kernel, bitwise.
-template <int D, int P, bool INTEG, bool XW, bool CH, int SPR>
-__global__ void __launch_bounds__(256, (P >= 4 ? 2 : (P >= 3 ? 4 : (P >= 2 ? 3 : 4)))) k_gather(
+//
+// EARLY (small systems of order <= 1): a launch that leaves SMs with a CTA or two is one chain of
+// latencies, so everything that does not need the field is read and drawn before the stencil (bond
+// partners, x_{n-1}, noise), at the registers of 2 CTAs per SM; and the kernel starts while the grid
+// passes before it end (the z pass lets its successors start only once the last step's kernels are done,
+// so positions and topology may be read before the wait).  us a step: 40^2 film 17.5 -> 16.1, 40^3 with
+// 157 CTAs 30.8 -> 29.8; 235 CTAs of order 4 70.7 -> 72.3 and 860 of order 1 with charges 130 -> 129.
+template <int D, int P, bool INTEG, bool XW, bool CH, int SPR, bool EARLY>
+__global__ void __launch_bounds__(256, EARLY ? 2 : (P >= 4 ? 2 : (P >= 3 ? 4 : (P >= 2 ? 3 : 4)))) k_gather(
     const float4* __restrict__ pos_in, float4* __restrict__ pos_io, float* __restrict__ noise,
     const int* __restrict__ bead_id, const int* __restrict__ bond_nbr, const int* __restrict__ bond_info,
     const float* __restrict__ charge, const float4* __restrict__ g4_all, const int* __restrict__ cta_sys,
     const SysDev* __restrict__ sysd, float* __restrict__ f_out, int f_sys, curandStateXORWOW_t* __restrict__ xw,
     int layout, unsigned long long* __restrict__ rho_fx_all, int spread_cap, int* status, int ahead, int blk_off) {
   static_assert(SPR == 0 || INTEG, "only integrating launches spread ahead");
+  static_assert(!EARLY || (INTEG && !XW && P <= 1), "early variants");
   const int s = cta_sys[blockIdx.x + blk_off];
   const SysDev& sd = sysd[s];
   const int i = (blockIdx.x + blk_off) * blockDim.x + threadIdx.x;
@@ -901,6 +915,7 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : (P >= 3 ? 4 : (P >= 2 ? 3 :
   const float q = (CH && C && t != kPadType) ? charge[i] : 0.f;
   bool sp = false;  // x (after the update) is spread ahead
   if (!active_at(sd, ahead)) {  // one system per CTA: every thread takes this branch together
+    if (EARLY) grid_wait();
     if (INTEG) pos_io[i] = p;  // inactive systems keep x_n through the buffer rotation
     if (SPR == 0) return;
     sp = t != kPadType && finite;  // held positions are spread too
@@ -944,6 +959,7 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : (P >= 3 ? 4 : (P >= 2 ? 3 :
       }
     }
   } else if (t != kPadType && !finite) {
+    if (EARLY) grid_wait();
     atomicOr(status, ST_NONFINITE_POS);
     if (SPR == 0) return;  // left in place; the host reports TILD_ERR_NAN
   } else if (t != kPadType) {
@@ -953,6 +969,22 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : (P >= 3 ? 4 : (P >= 2 ? 3 :
     const float4* g4 = g4_all + sd.g4_0;
 
     float f[3] = {0.f, 0.f, 0.f};
+    int info = 0, nb = 0, bid = 0, ig0 = -1;
+    float4 pj[3], po = make_float4(0.f, 0.f, 0.f, 0.f);
+    float on0[3] = {0.f, 0.f, 0.f}, z0[3] = {0.f, 0.f, 0.f};
+    if (EARLY) {
+      info = bond_info[i];
+      nb = info & 3;
+      bid = bead_id[i];
+      po = pos_io[i];
+#pragma unroll
+      for (int d = 0; d < D; d++) on0[d] = noise[3 * (long long)i + d];
+#pragma unroll
+      for (int bb = 0; bb < 3; bb++)
+        if (bb < nb) pj[bb] = pos_in[bond_nbr[3 * i + bb]];
+      ig0 = __ffs(sd.type_mask[t]) - 1;
+      if (ig0 >= 0) philox_normal3(sd.seed, (uint32_t)bid, sd.step + ahead + 1, (uint32_t)ig0, z0);
+    }
     {
       float W[3][P + 1];
       int idx[3][P + 1];
@@ -964,6 +996,10 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : (P >= 3 ? 4 : (P >= 2 ? 3 :
       }
       int o[3][P + 1];
       field_offsets<D, P>(idx, layout, g, o);
+      if (EARLY) {
+        grid_wait();
+        g4 = after_wait(g4);
+      }
       if (CH && C && q != 0.f) {
         float e[3] = {0.f, 0.f, 0.f};
         gather4<D, P>(g4 + (long long)T * Mb, W, o, e);
@@ -972,24 +1008,27 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : (P >= 3 ? 4 : (P >= 2 ? 3 :
       }
       gather4<D, P>(g4 + (long long)t * Mb, W, o, f);
     }
-    // bond partners and x_{n-1} are read after the stencil: held across it they cost the stencil
-    // registers (measured 1-4 % slower gathers)
-    const int info = bond_info[i];
-    const int nb = info & 3;
-    float4 pj[3];
+    if (!EARLY) {
+      // bond partners and x_{n-1} are read after the stencil: held across it they cost the stencil
+      // registers (measured 1-4 % slower gathers)
+      info = bond_info[i];
+      nb = info & 3;
 #pragma unroll
-    for (int bb = 0; bb < 3; bb++)
-      if (bb < nb) pj[bb] = pos_in[bond_nbr[3 * i + bb]];
-    const int bid = bead_id[i];
-    float4 po = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (INTEG) po = pos_io[i];  // x_{n-1} (GJF xo)
-    bead_epilogue<D, INTEG, XW>(i, p, t, x, f, sd, g, info, nb, pj, bid, po, noise, pos_io, f_out, f_sys, s, xw, ahead);
+      for (int bb = 0; bb < 3; bb++)
+        if (bb < nb) pj[bb] = pos_in[bond_nbr[3 * i + bb]];
+      bid = bead_id[i];
+      if (INTEG) po = pos_io[i];  // x_{n-1} (GJF xo)
+    }
+    bead_epilogue<D, INTEG, XW, EARLY>(i, p, t, x, f, sd, g, info, nb, pj, bid, po, noise, pos_io, f_out, f_sys, s, xw, ahead,
+                                       on0, z0, ig0);
     if (SPR != 0) {
       sp = isfinite(x[0]) && isfinite(x[1]) && (D == 2 || isfinite(x[2]));
       if (!sp) atomicOr(status, ST_NONFINITE_POS);
     }
   } else if (SPR == 0) {
     return;  // padding slot
+  } else if (EARLY) {
+    grid_wait();
   }
   if constexpr (SPR == 1) cta_spread_box<D, P, CH>(sp, x, t, q, sd, rho_fx_all + sd.grid0, spread_cap, status);
   if constexpr (SPR == 2)
@@ -1269,6 +1308,19 @@ void launch_gather_k(tild_ctx* c, float* f_out, int f_sys, BeadRange r) {
         c->cta_bead, c->d_sys, f_out, f_sys, c->xorwow, c->gather_cap, c->d_status, c->ahead, r.off);
     return;
   }
+  if constexpr (I && !X && P <= 1) {
+    const bool ahead = tild_spreads_ahead(c, true);
+    if (r.n < 296) {  // 2 CTAs per SM
+      auto early = [&](auto* kernel, unsigned long long* rho_fx) {
+        tild_launch_early(kernel, r.n, kTile, 0, kCarveout, r.st, c->pos[c->cur], c->pos[c->cur ^ 1], c->noise, c->bead_id,
+                          c->bond_nbr, c->bond_info, c->charge, c->g4, c->cta_bead, c->d_sys, f_out, f_sys, c->xorwow,
+                          c->field_layout, rho_fx, 0, c->d_status, c->ahead, r.off);
+      };
+      if (ahead) early(k_gather<D, P, I, X, CH, 2, true>, c->rho_fx);
+      else early(k_gather<D, P, I, X, CH, 0, true>, nullptr);
+      return;
+    }
+  }
   if constexpr (I) {
     if (tild_spreads_ahead(c, true)) {
       if constexpr (P >= 2) {
@@ -1276,11 +1328,11 @@ void launch_gather_k(tild_ctx* c, float* f_out, int f_sys, BeadRange r) {
           static std::atomic<unsigned long long> attr_devices{0};  // one bit per device with the attribute set
           const unsigned long long bit = 1ull << (c->device & 63);
           if (!(attr_devices.load() & bit)) {
-            cudaFuncSetAttribute(k_gather<D, P, I, X, CH, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(k_gather<D, P, I, X, CH, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(sizeof(int) * 12288));
             attr_devices.fetch_or(bit);
           }
-          k_gather<D, P, I, X, CH, 1><<<r.n, kTile, sizeof(int) * (size_t)c->spread_cap, r.st>>>(
+          k_gather<D, P, I, X, CH, 1, false><<<r.n, kTile, sizeof(int) * (size_t)c->spread_cap, r.st>>>(
               c->pos[c->cur], c->pos[c->cur ^ 1], c->noise, c->bead_id, c->bond_nbr, c->bond_info, c->charge, c->g4,
               c->cta_bead, c->d_sys, f_out, f_sys, c->xorwow, c->field_layout, c->rho_fx, c->spread_cap,
               c->d_status, c->ahead, r.off);
@@ -1291,12 +1343,12 @@ void launch_gather_k(tild_ctx* c, float* f_out, int f_sys, BeadRange r) {
         static std::atomic<unsigned long long> attr_devices2{0};
         const unsigned long long bit = 1ull << (c->device & 63);
         if (!(attr_devices2.load() & bit)) {
-          cudaFuncSetAttribute(k_gather<D, P, I, X, CH, 2>, cudaFuncAttributePreferredSharedMemoryCarveout,
+          cudaFuncSetAttribute(k_gather<D, P, I, X, CH, 2, false>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                cudaSharedmemCarveoutMaxL1);
           attr_devices2.fetch_or(bit);
         }
       }
-      k_gather<D, P, I, X, CH, 2><<<r.n, kTile, 0, r.st>>>(  // spread ahead by global atomics
+      k_gather<D, P, I, X, CH, 2, false><<<r.n, kTile, 0, r.st>>>(  // spread ahead by global atomics
           c->pos[c->cur], c->pos[c->cur ^ 1], c->noise, c->bead_id, c->bond_nbr, c->bond_info, c->charge, c->g4,
           c->cta_bead, c->d_sys, f_out, f_sys, c->xorwow, c->field_layout, c->rho_fx, 0, c->d_status, c->ahead, r.off);
       return;
@@ -1307,7 +1359,7 @@ void launch_gather_k(tild_ctx* c, float* f_out, int f_sys, BeadRange r) {
     static std::atomic<unsigned long long> attr_devices{0};  // one bit per device with the attribute set
     const unsigned long long bit = 1ull << (c->device & 63);
     if (!(attr_devices.load() & bit)) {
-      cudaFuncSetAttribute(k_gather<D, P, I, X, CH, 0>, cudaFuncAttributePreferredSharedMemoryCarveout,
+      cudaFuncSetAttribute(k_gather<D, P, I, X, CH, 0, false>, cudaFuncAttributePreferredSharedMemoryCarveout,
                            cudaSharedmemCarveoutMaxL1);
       attr_devices.fetch_or(bit);
     }
@@ -1320,11 +1372,11 @@ void launch_gather_k(tild_ctx* c, float* f_out, int f_sys, BeadRange r) {
     static std::atomic<unsigned long long> attr_devices{0};  // one bit per device with the attribute set
     const unsigned long long bit = 1ull << (c->device & 63);
     if (!(attr_devices.load() & bit)) {
-      cudaFuncSetAttribute(k_gather<D, P, I, X, CH, 0>, cudaFuncAttributePreferredSharedMemoryCarveout, 40);
+      cudaFuncSetAttribute(k_gather<D, P, I, X, CH, 0, false>, cudaFuncAttributePreferredSharedMemoryCarveout, 40);
       attr_devices.fetch_or(bit);
     }
   }
-  k_gather<D, P, I, X, CH, 0><<<r.n, kTile, 0, r.st>>>(
+  k_gather<D, P, I, X, CH, 0, false><<<r.n, kTile, 0, r.st>>>(
       c->pos[c->cur], c->pos[c->cur ^ 1], c->noise, c->bead_id, c->bond_nbr, c->bond_info, c->charge, c->g4,
       c->cta_bead, c->d_sys, f_out, f_sys, c->xorwow, c->field_layout, nullptr, 0, c->d_status, c->ahead, r.off);
 }
