@@ -52,6 +52,21 @@ __global__ void k_pack_noise(const float* __restrict__ src, const int* __restric
   for (int d = 0; d < 3; d++) noise[3 * (long long)s + d] = (src && d < D) ? src[(long long)b * D + d] : 0.f;
 }
 
+// A whole new state (x_{n-1} = x, no previous noise) in one launch; nothing changes when the check
+// flagged a value.
+__global__ void k_pack_state(const float* __restrict__ x, const int* __restrict__ types, const int* __restrict__ slot_of,
+                             int ns, int D, const int* __restrict__ bad, float4* __restrict__ pos, float4* __restrict__ prev,
+                             float* __restrict__ noise) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= ns || *bad) return;
+  const int s = slot_of[b];
+  const float* xb = x + (long long)b * D;
+  const float4 p = make_float4(xb[0], xb[1], D == 3 ? xb[2] : 0.f, __int_as_float(types[b] & 0xff));
+  pos[s] = p;
+  prev[s] = p;
+  for (int d = 0; d < 3; d++) noise[3 * (long long)s + d] = 0.f;
+}
+
 __global__ void k_unpack_pos(const float4* __restrict__ pos, const int* __restrict__ bead_id, int n, int D,
                              float* __restrict__ x) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -115,6 +130,7 @@ void free_all(tild_ctx* c) {
     }
   for (auto& ge : c->graphs) cudaGraphExecDestroy(ge.exec);
   c->graphs.clear();
+  if (c->h_status) cudaFreeHost(c->h_status);
   tild_sort_free(c);
   tild_fft_free(c);
   for (cudaStream_t a : c->aux) cudaStreamDestroy(a);
@@ -558,6 +574,10 @@ int engine_create(const tild_config* cfgs, int nsys, int device, tild_ctx* c, co
   rc = rc ? rc : dalloc(c, &c->kk, (size_t)kd, "k vectors");
   rc = rc ? rc : dalloc(c, &c->xfer, (size_t)maxns * 3, "transfer buffer");
   rc = rc ? rc : dalloc(c, &c->d_status, 2, "status");  // [0] status word, [1] input check flag
+  if (!rc && cudaMallocHost(&c->h_status, 2 * sizeof(int)) != cudaSuccess) {
+    cudaGetLastError();
+    return set_err(c, TILD_ERR_OOM, "page-locked memory for the status word");
+  }
   rc = rc ? rc : dalloc(c, &c->d_sys, (size_t)nsys, "system descriptors");
   rc = rc ? rc : dalloc(c, &c->cta_bead, tb.size(), "lookup");
   rc = rc ? rc : dalloc(c, &c->cta_spec, tspec.size(), "lookup");
@@ -700,16 +720,26 @@ int sys_set_state(tild_ctx* c, int s, const float* x, const float* xo, const flo
   const int* ty = c->types_dev + h.bead0;
   if (tild_check(c, cudaMemcpyAsync(c->xfer, x, n * 4, cudaMemcpyHostToDevice, st), "upload x")) return TILD_ERR_CUDA;
   // the positions are checked on the device before anything of the current state changes
+  const bool fresh = !xo && !prev_noise && !c->rho_ahead && !c->xorwow;
   {
-    int bad = 0;
     if (tild_check(c, cudaMemsetAsync(c->d_status + 1, 0, sizeof(int), st), "clear check flag")) return TILD_ERR_CUDA;
     k_check_finite<<<std::min<unsigned>(nblk((long long)n, 256), 1184), 256, 0, st>>>(c->xfer, (long long)n,
                                                                                         c->d_status + 1);
     c->launches++;
-    if (tild_check(c, cudaMemcpyAsync(&bad, c->d_status + 1, sizeof(int), cudaMemcpyDeviceToHost, st), "check flag") ||
+    if (fresh) {  // the packing itself looks at the flag: one wait for both
+      k_pack_state<<<nb, 256, 0, st>>>(c->xfer, ty, so, h.ns, h.D, c->d_status + 1, c->pos[c->cur], c->pos[c->cur ^ 1], c->noise);
+      c->launches++;
+    }
+    if (tild_check(c, cudaMemcpyAsync(c->h_status + 1, c->d_status + 1, sizeof(int), cudaMemcpyDeviceToHost, st), "check flag") ||
         tild_check(c, cudaStreamSynchronize(st), "sync check"))
       return TILD_ERR_CUDA;
-    if (bad) return set_err(c, TILD_ERR_NAN, "non-finite position in tild_set_state");
+    if (c->h_status[1]) return set_err(c, TILD_ERR_NAN, "non-finite position in tild_set_state");
+  }
+  if (fresh) {
+    c->steps_since_sort = c->sort_interval;  // sort before the next step
+    h.state_set = true;
+    h.have_forces = false;
+    return TILD_OK;
   }
   if (tild_drop_ahead(c)) return TILD_ERR_CUDA;
   k_pack_pos<<<nb, 256, 0, st>>>(c->xfer, ty, so, h.ns, h.D, c->pos[c->cur]);
@@ -1376,10 +1406,10 @@ int tild_check_fft(tild_ctx* c, cufftResult r, const char* what) {
 }
 
 int tild_poll_status(tild_ctx* c) {
-  int st = 0;
-  if (tild_check(c, cudaMemcpyAsync(&st, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "status") ||
+  if (tild_check(c, cudaMemcpyAsync(c->h_status, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "status") ||
       tild_check(c, cudaStreamSynchronize(c->stream), "sync"))
     return TILD_ERR_CUDA;
+  const int st = *c->h_status;
   if (st & ST_NONFINITE_POS) return set_err(c, TILD_ERR_NAN, "non-finite bead position");
   if (st & ST_INDEX_RANGE) return set_err(c, TILD_ERR_BAD_INPUT, "bead position outside [-L, 2L): grid index out of range");
   if (st & ST_NLIST_OVERFLOW) {

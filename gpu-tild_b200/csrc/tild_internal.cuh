@@ -230,6 +230,7 @@ struct tild_ctx {
   int red_cap = 0;
   float* xfer = nullptr;                 // staging for host transfers, >= 3 * max ns floats
   int* d_status = nullptr;               // [0] status word, [1] input check flag
+  int* h_status = nullptr;               // page-locked copy
 
   // spatial sort (tild_sort.cu)
   unsigned* sort_keys = nullptr;
@@ -251,6 +252,7 @@ struct tild_ctx {
   int sort_cell_bits = 0;
   int sort_interval = 0;                 // 0: never
   int64_t steps_since_sort = 0;
+  int64_t evals_since_sort = 1 << 20;    // force-only evaluations; none sorted yet
   long long sorts = 0;
   int spread_cap = 0;                    // shared-memory 32-bit words of the tiled spread
 

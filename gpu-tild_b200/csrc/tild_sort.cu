@@ -197,6 +197,7 @@ int tild_sort_beads(tild_ctx* c) {
   c->launches += 2;
   tild_sort_swap_buffers(c);
   c->steps_since_sort = 0;
+  c->evals_since_sort = 0;
   c->sorts++;
   return tild_check(c, cudaGetLastError(), "sort") ? TILD_ERR_CUDA : TILD_OK;
 }
