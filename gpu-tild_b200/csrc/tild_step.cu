@@ -365,35 +365,6 @@ __global__ void k_fix_to_pairs(unsigned long long* __restrict__ fx, float2* __re
   a[M] = 0ull;
 }
 
-// Both conversions over grid blocks [blk_off, ..) of any shapes in one launch: a CTA takes 256 nodes of
-// one system and all its channels (an ensemble of 25 grid shapes converted shape by shape spent
-// 100 us on 25 launches of 4 us).
-__global__ void __launch_bounds__(256) k_fix_nodes(unsigned long long* __restrict__ fx_all, float* __restrict__ rho_all,
-                                                   const int* __restrict__ cta_sys, const int* __restrict__ blk0,
-                                                   const SysDev* __restrict__ sysd, int blk_off) {
-  const int blk = blockIdx.x + blk_off, s = cta_sys[blk];
-  const SysDev& sd = sysd[s];
-  const long long M = sd.g.M, m = (long long)(blk - blk0[s]) * blockDim.x + threadIdx.x;
-  if (m >= M) return;
-  const int nch = sd.T + sd.C;
-  const bool paired = sd.fwd_packed;
-  unsigned long long* fx = fx_all + sd.grid0 + m;
-  float* rho = rho_all + sd.grid0;
-  for (int c = 0; c < nch; c += 2) {
-    const bool two = c + 1 < nch;
-    const long long va = (long long)fx[c * M], vb = two ? (long long)fx[(c + 1) * M] : 0;
-    fx[c * M] = 0ull;
-    if (two) fx[(c + 1) * M] = 0ull;
-    const float a = (float)((double)va * kInvFix), b = (float)((double)vb * kInvFix);
-    if (paired) {
-      reinterpret_cast<float2*>(rho + c * M)[m] = make_float2(a, b);
-    } else {
-      rho[c * M + m] = a;
-      if (two) rho[(c + 1) * M + m] = b;
-    }
-  }
-}
-
 // paired density spectra -> per-channel half spectra (the R2C layout, for the observables and S(k)):
 // one thread per half-spectrum point, every pair of the system
 __global__ void k_unpack_half(const float2* __restrict__ z, float2* __restrict__ half, int npairs, Geom g, int D) {
@@ -1605,21 +1576,18 @@ int tild_run_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys) {
   for (const Bucket& b : c->buckets) any_lib = any_lib || !b.own;
   if (!any_lib) return tild_finish_forces(c, integrate, f_bead, f_sys, true, false);
   // runs of neighbouring shapes that take the library, in one launch each
-  struct Range { int g0, ng, s0, ns; };
+  struct Range { int s0, ns; };
   std::vector<Range> runs;
   bool open = false;
   for (const Bucket& b : c->buckets) {
     if (b.own) { open = false; continue; }
-    if (!open) runs.push_back({b.cta_grid0, 0, b.cta_spec0, 0});
+    if (!open) runs.push_back({b.cta_spec0, 0});
     open = true;
-    runs.back().ng += b.n_cta_grid;
     runs.back().ns += b.n_cta_spec;
   }
   tild_mark(c, STAGE_ZERO);
-  for (const Range& r : runs) {
-    k_fix_nodes<<<r.ng, 256, 0, c->stream>>>(c->rho_fx, c->rho, c->cta_grid, c->cta_grid + c->n_cta_grid, c->d_sys, r.g0);
-    c->launches++;
-  }
+  for (const Bucket& b : c->buckets)
+    if (!b.own) launch_fix(c, b, c->stream);
   if (tild_check(c, cudaGetLastError(), "spread")) return TILD_ERR_CUDA;
   tild_mark(c, STAGE_R2C);
   if (fork(c)) return TILD_ERR_CUDA;
