@@ -889,6 +889,208 @@ __global__ void __launch_bounds__(kThreadsX, kMinCtasX) k_fft_x_inv(const float2
   }
 }
 
+// ---- small planes: x and y passes in one kernel each -------------------------------------------------
+// A plane of up to kPlanePoints points fits in shared memory twice, so a CTA converts and transforms a
+// whole z plane of a pair, and takes one field of a plane back through y and x to its component of the
+// float4 nodes (4-byte stores in place of 16-byte ones).  Two kernels less on the path of a step whose
+// passes take 4 us each, us a step with and without: 40^3 diblock 28.4 / 29.7, 45^3 melt 51.5 / 54.0,
+// 33x52x75 lamella 67.2 / 70.9, 8 slots of 24^3 to 45^3 60.9 / 64.4.  512 threads take every stage of a
+// plane in one round; the inverse of more than 2 planes' fields per SM is better off with twice the CTAs
+// (the 8 slots: 16.8 against 20.7 us, 48^3: 33.3 against 30.3 a step).
+constexpr int kPlanePoints = 2304, kThreadsPlane = 512;
+__host__ __device__ inline int plane_exchange(int nx, int ny, int r1x, int r2x) {  // complex values of the exchange
+  const int rows = ny * r1x * (r2x | 1);
+  return rows > nx * ny ? rows : nx * ny;
+}
+
+__global__ void __launch_bounds__(kThreadsPlane, 1024 / kThreadsPlane)
+    k_fft_plane_fwd(unsigned long long* __restrict__ fx, float* __restrict__ rho, float2* __restrict__ zk,
+                    const float2* __restrict__ twid, const int2* __restrict__ blocks, const SysDev* __restrict__ sysd,
+                    int write_rho, int ahead, int blk_off) {
+  extern __shared__ __align__(16) float2 ex[];
+  const int2 bk = blocks[blockIdx.x + blk_off];
+  const SysDev& sd = sysd[bk.x];
+  const Lines g(sd.g, 3);
+  const int nx = g.nx, ny = g.ny, npt = nx * ny;
+  const int R1 = sd.fft_r1[0], R2 = sd.fft_r2[0], R2p = R2 | 1, Y1 = sd.fft_r1[1], Y2 = sd.fft_r2[1];
+  const float2 *twr = twid + sd.fft_tw[0] + sd.fft_twr, *twy = twid + sd.fft_tw[1];
+  const int p = bk.y / g.nz, plane = bk.y - p * g.nz;
+  const bool two = 2 * p + 1 < sd.T + sd.C, paired = sd.fwd_packed;
+  float2* in = ex + plane_exchange(nx, ny, R1, R2);
+  unsigned long long* a = fx + sd.grid0 + 2 * (long long)p * g.M + (long long)plane * npt;
+  float* ra = rho + sd.grid0 + 2 * (long long)p * g.M;
+  float2* rp = reinterpret_cast<float2*>(ra) + (long long)plane * npt;
+  ra += (long long)plane * npt;
+  grid_launch_next();
+  grid_wait();
+  const bool act = active_at(*after_wait(&sd), ahead);
+  a = after_wait(a);
+  unsigned long long* b = a + g.M;
+  for (int i0 = threadIdx.x; i0 < npt; i0 += kXBatch * kThreadsPlane) {
+    long long va[kXBatch], vb[kXBatch];
+#pragma unroll
+    for (int q = 0; q < kXBatch; q++) {
+      const int i = i0 + q * kThreadsPlane;
+      va[q] = i < npt ? (long long)a[i] : 0;
+      vb[q] = two && i < npt ? (long long)b[i] : 0;
+    }
+#pragma unroll
+    for (int q = 0; q < kXBatch; q++) {
+      const int i = i0 + q * kThreadsPlane;
+      if (i >= npt) break;
+      a[i] = 0ull;
+      if (two) b[i] = 0ull;
+      const float2 v = make_float2(__ll2float_rn(va[q]) * 0x1p-32f, __ll2float_rn(vb[q]) * 0x1p-32f);
+      if (write_rho) {
+        if (paired) {
+          rp[i] = v;
+        } else {
+          ra[i] = v.x;
+          if (two) ra[g.M + i] = v.y;
+        }
+      }
+      in[i] = v;
+    }
+  }
+  if (!act) return;  // one system per CTA
+  __syncthreads();
+  const FastDiv dj(R2), dk(R1), dx(nx);
+  with_radix(R1, [&](auto rc) {
+    constexpr int R = decltype(rc)::value;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < ny * R2; i += kThreadsPlane) {
+      const int line = dj.div(i), j = i - line * R2, from = here(R2), to = here(R2p);
+      const float2* s = in + line * nx + j;
+      float2 v[R];
+#pragma unroll
+      for (int n = 0; n < R; n++) v[n] = s[n * from];
+      dft_twiddle_rows<R>(v, j, R2, twr);
+      float2* e = ex + line * R * R2p + j;
+#pragma unroll
+      for (int k = 0; k < R; k++) e[k * to] = v[k];
+    }
+  });
+  __syncthreads();
+  second_stage<false>(threadIdx.x, kThreadsPlane, ny * R1, R1, R2, 1, twr, [&](int q) { return ex + q * R2p; },
+                      [&](int q) {
+                        const int line = dk.div(q);
+                        return in + line * nx + (q - line * R1);
+                      },
+                      [&](float2* d, int k2, float2 v) { d[k2 * R1] = v; });
+  __syncthreads();
+  with_radix(Y1, [&](auto rc) {
+    constexpr int R = decltype(rc)::value;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < nx * Y2; i += kThreadsPlane) {
+      const int j = dx.div(i), from = here(Y2 * nx), to = here(nx);
+      const float2* s = in + i;  // row j, column i - j nx
+      float2 v[R];
+#pragma unroll
+      for (int n = 0; n < R; n++) v[n] = s[n * from];
+      dft_twiddle<R>(v, j, twy);
+      float2* e = ex + j * (R - 1) * nx + i;
+#pragma unroll
+      for (int k = 0; k < R; k++) e[k * to] = v[k];
+    }
+  });
+  __syncthreads();
+  float2* z = zk + sd.zk0 + (long long)p * g.M + (long long)plane * npt;
+  const unsigned step = Y1 * nx * sizeof(float2);
+  second_stage<false>(threadIdx.x, kThreadsPlane, nx * Y1, Y1, Y2, Y1 * nx, twy, [&](int q) { return ex + q; },
+                      [&](int q) { return Run(z + q, step); }, [](const Run& d, int k2, float2 v) { d[k2] = v; });
+}
+
+struct PlaneValue {
+  float2* p;
+  float k;
+};
+struct NodeRun {
+  float *a, *b;
+  int x;
+};
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
+    k_fft_plane_inv(const float2* __restrict__ gk, float4* __restrict__ g4_all, const float* __restrict__ kd_all,
+                    const float2* __restrict__ twid, const int2* __restrict__ blocks, const SysDev* __restrict__ sysd,
+                    int layout, int ahead, int blk_off) {
+  extern __shared__ __align__(16) float2 ex[];
+  const int2 bk = blocks[blockIdx.x + blk_off];
+  const SysDev& sd = sysd[bk.x];
+  const Lines g(sd.g, 3);
+  const int nx = g.nx, ny = g.ny, npt = nx * ny;
+  const int R1 = sd.fft_r1[0], R2 = sd.fft_r2[0], R2p = R2 | 1, Y1 = sd.fft_r1[1], Y2 = sd.fft_r2[1];
+  const float2 *twr = twid + sd.fft_tw[0] + sd.fft_twr, *twy = twid + sd.fft_tw[1];
+  const int f = bk.y % 3, r = bk.y / 3, p = r / g.nz, plane = r - p * g.nz;  // f: x, y, z derivative
+  float2* pl = ex + plane_exchange(nx, ny, R1, R2);
+  const float2* src = gk + sd.gkp0 + (long long)p * 3 * g.M + (f == 2 ? 2 * g.M : 0) + (long long)plane * npt;
+  const float *kx = kd_all + sd.kd0, *ky = kx + nx;
+  const FastDiv dj(R2), dk(R1), dx(nx);
+  grid_launch_next();
+  grid_wait();
+  if (!active_at(*after_wait(&sd), ahead)) return;
+  src = after_wait(src);
+  with_radix(Y1, [&](auto rc) {
+    constexpr int R = decltype(rc)::value;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < nx * Y2; i += THREADS) {
+      const int j = dx.div(i), to = here(nx);
+      const Run s(src + i, Y2 * nx * sizeof(float2));
+      float2 v[R];
+#pragma unroll
+      for (int n = 0; n < R; n++) v[n] = swapped(s[n]);
+      if (f == 1) {
+#pragma unroll
+        for (int n = 0; n < R; n++) {  // swapped(-i k P) from swapped(P)
+          const float k = __ldg(ky + n * Y2 + j);
+          v[n] = make_float2(-k * v[n].y, k * v[n].x);
+        }
+      }
+      dft_twiddle<R>(v, j, twy);
+      float2* e = ex + j * (R - 1) * nx + i;
+#pragma unroll
+      for (int k = 0; k < R; k++) e[k * to] = v[k];
+    }
+  });
+  __syncthreads();
+  second_stage<false>(threadIdx.x, THREADS, nx * Y1, Y1, Y2, Y1 * nx, twy, [&](int q) { return ex + q; },
+                      [&](int q) { return PlaneValue{pl + q, f ? 0.f : __ldg(kx + (q - dx.div(q) * nx))}; },
+                      [&](const PlaneValue& d, int k2, float2 v) {
+                        d.p[k2 * (Y1 * nx)] = f ? v : make_float2(-d.k * v.y, d.k * v.x);
+                      });
+  __syncthreads();
+  with_radix(R1, [&](auto rc) {
+    constexpr int R = decltype(rc)::value;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < ny * R2; i += THREADS) {
+      const int line = dj.div(i), j = i - line * R2, from = here(R2), to = here(R2p);
+      const float2* s = pl + line * nx + j;
+      float2 v[R];
+#pragma unroll
+      for (int n = 0; n < R; n++) v[n] = s[n * from];
+      dft_twiddle_rows<R>(v, j, R2, twr);
+      float2* e = ex + line * R * R2p + j;
+#pragma unroll
+      for (int k = 0; k < R; k++) e[k * to] = v[k];
+    }
+  });
+  __syncthreads();
+  float* ga = reinterpret_cast<float*>(g4_all + sd.g4_0 + 2 * (long long)p * sd.Mb) + f;
+  const bool two = 2 * p + 1 < sd.T + sd.C, linear = layout == TILD_FIELD_LINEAR;
+  const long long second = 4 * sd.Mb;
+  const int zoff = linear ? plane * npt : tild_field_off(layout, 2, plane, sd.g);
+  second_stage<false>(threadIdx.x, THREADS, ny * R1, R1, R2, 1, twr, [&](int q) { return ex + q * R2p; },
+                      [&](int q) {
+                        const int line = dk.div(q), row = zoff + (linear ? line * nx : tild_field_off(layout, 1, line, sd.g));
+                        float* at = ga + 4ll * row;
+                        return NodeRun{at, at + second, q - line * R1};
+                      },
+                      [&](const NodeRun& d, int k2, float2 v) {  // v is swapped(result): the real part is channel 2p's
+                        const int x = d.x + R1 * k2, o = 4 * (linear ? x : ((x >> 2) << 6) | (x & 3));
+                        d.a[o] = v.y;
+                        if (two) d.b[o] = v.x;
+                      });
+}
+
 // fieldphase on the interleaved field: type a gets +rho_a f_r, type b -rho_b f_r (planar densities)
 __global__ void k_fieldphase_nodes(float4* __restrict__ g4, long long Mb, const float* __restrict__ rho,
                                    const float* __restrict__ fr, int a, int b, Geom g, int D, int layout) {
@@ -985,6 +1187,14 @@ int tild_fft_setup(tild_ctx* c) {
     for (int s : b.systems)
       if (b.own) points += (c->sys[s].T + c->sys[s].C + 1) / 2 * c->sys[s].g.M;
   c->fft_points = (int)std::min(1024ll, std::max(256ll, points / 592));
+  // small planes without direct transforms in x or y
+  c->fft_plane = D == 3;
+  for (const Bucket& b : c->buckets) {
+    int r1, r2;
+    if (!b.own) continue;
+    c->fft_plane = c->fft_plane && b.nx[0] * b.nx[1] <= kPlanePoints;
+    for (int a = 0; a < 2 && c->fft_plane; a++) c->fft_plane = split_length(b.nx[a], &r1, &r2) && r2 <= 16;
+  }
   c->fft_wide = points >= 16 * 32 * 592;  // the y inverse pass still has some CTAs of 16 columns for every SM
   std::vector<int2> tab[5];
   long long ztotal = 0;
@@ -1031,15 +1241,20 @@ int tild_fft_setup(tild_ctx* c) {
         const int zcols = z_columns(nx, ny);
         const int ltx = rows_per_cta(nx, c->fft_points);
         const long long rows = (long long)ny * nz, cols = (long long)nx * nz;
-        const int nblocks[5] = {np * (int)nblk(rows, ltx), np * (int)nblk(cols, kColsFwd), (int)nblk(zcols, kColsZ),
+        int nblocks[5] = {np * (int)nblk(rows, ltx), np * (int)nblk(cols, kColsFwd), (int)nblk(zcols, kColsZ),
                                 np * (int)nblk(cols, c->fft_wide ? 16 : 8), np * (int)nblk(rows, ltx)};
         d.zt0 = ztotal;
         if (h.T <= TILD_MAXT_FAST) ztotal += (long long)nblocks[2] * (h.T * (h.T + 1) / 2 + h.C) * nz * kColsZ;
         const int rx2 = d.fft_r2[0], row = d.fft_r1[0] * (rx2 | 1);
-        const size_t smem[5] = {sizeof(float2) * ltx * (row + nx), sizeof(float2) * kColsFwd * ny, z_smem(nz, h.T, h.C),
+        size_t smem[5] = {sizeof(float2) * ltx * (row + nx), sizeof(float2) * kColsFwd * ny, z_smem(nz, h.T, h.C),
                                 sizeof(float2) * (c->fft_wide ? 16 : 3 * 8) * (d.fft_r1[1] | 1) * d.fft_r2[1], (rx2 > 16 ? 2 : 1) * D * sizeof(float2) * ltx * row};
+        if (c->fft_plane) {
+          nblocks[0] = np * nz;
+          nblocks[4] = 3 * np * nz;
+          smem[0] = smem[4] = sizeof(float2) * (nx * ny + plane_exchange(nx, ny, d.fft_r1[0], d.fft_r2[0]));
+        }
         for (int k = 0; k < 5; k++) {
-          if (D == 2 && (k == 1 || k == 3)) continue;
+          if ((D == 2 || c->fft_plane) && (k == 1 || k == 3)) continue;
           auto& pa = c->fft_pass[k];
           pa.smem = std::max(pa.smem, smem[k]);
           for (int q = 0; q < nblocks[k]; q++) tab[k].push_back(make_int2(s, q));
@@ -1061,7 +1276,7 @@ int tild_fft_setup(tild_ctx* c) {
       return TILD_ERR_CUDA;
   }
   auto both = [](auto* regular, auto* direct) { return allow_smem(regular) && allow_smem(direct); };
-  const bool okattr = allow_smem(k_fft_x_fwd) && both(k_fft_y_fwd<false>, k_fft_y_fwd<true>) &&
+  const bool okattr = allow_smem(k_fft_plane_fwd) && both(k_fft_plane_inv<256>, k_fft_plane_inv<512>) && allow_smem(k_fft_x_fwd) && both(k_fft_y_fwd<false>, k_fft_y_fwd<true>) &&
                       both(k_fft_z_kmul<false>, k_fft_z_kmul<true>) && both(k_fft_y_inv<8, false>, k_fft_y_inv<8, true>) &&
                       both(k_fft_y_inv<16, false>, k_fft_y_inv<16, true>) && both(k_fft_x_inv<false>, k_fft_x_inv<true>);
   if (!okattr) {
@@ -1116,10 +1331,15 @@ int tild_fft_run(tild_ctx* c, const Bucket* b, bool integrate, bool active, cuda
   const int wr = !integrate || c->last_of_call || !c->fields.empty(), ahead = c->ahead;
   const bool* dir = b ? b->fft_direct : c->fft_direct;
   if (!b) tild_mark(c, STAGE_ZERO);
-  tild_launch_early(k_fft_x_fwd, n[0], kThreads, pa[0].smem, kCarveout, st, c->rho_fx, c->rho, zk, c->fft_twid, pa[0].blocks, c->d_sys, c->D, c->fft_points, wr, ahead, off[0]);
+  if (c->fft_plane)
+    tild_launch_early(k_fft_plane_fwd, n[0], kThreadsPlane, pa[0].smem, kCarveout, st, c->rho_fx, c->rho, zk, c->fft_twid, pa[0].blocks,
+                      c->d_sys, wr, ahead, off[0]);
+  else
+    tild_launch_early(k_fft_x_fwd, n[0], kThreads, pa[0].smem, kCarveout, st, c->rho_fx, c->rho, zk, c->fft_twid, pa[0].blocks, c->d_sys, c->D, c->fft_points, wr, ahead, off[0]);
   c->launches++;
   if (!active) return tild_check(c, cudaGetLastError(), "grid passes");  // no system of the shape moves: densities only
-  if (c->D == 3) {
+  const bool columns = c->D == 3 && !c->fft_plane;
+  if (columns) {
     if (!b) tild_mark(c, STAGE_R2C);
     tild_launch_early(dir[1] ? k_fft_y_fwd<true> : k_fft_y_fwd<false>, n[1], kThreads, pa[1].smem, kCarveout, st, zk, c->fft_twid, pa[1].blocks, c->d_sys, ahead, off[1]);
     c->launches++;
@@ -1127,7 +1347,7 @@ int tild_fft_run(tild_ctx* c, const Bucket* b, bool integrate, bool active, cuda
   if (!b) tild_mark(c, STAGE_KMUL);
   tild_launch_early(dir[2] ? k_fft_z_kmul<true> : k_fft_z_kmul<false>, n[2], kThreadsZ, pa[2].smem, kCarveout, st, zk, gk, c->ztab, c->utab, c->ctab, c->kd, c->fft_twid, pa[2].blocks, c->d_sys,
               c->D, (int)integrate, ahead, off[2]);
-  if (c->D == 3) {
+  if (columns) {
     if (!b) tild_mark(c, STAGE_C2R);
     if (c->fft_wide)
       tild_launch_early(dir[1] ? k_fft_y_inv<16, true> : k_fft_y_inv<16, false>, n[3], 128, pa[3].smem, kCarveout, st, gk, c->kd, c->fft_twid, pa[3].blocks, c->d_sys, ahead, off[3]);
@@ -1136,7 +1356,11 @@ int tild_fft_run(tild_ctx* c, const Bucket* b, bool integrate, bool active, cuda
     c->launches++;
   }
   if (!b) tild_mark(c, STAGE_INTERLEAVE);
-  tild_launch_early(dir[0] ? k_fft_x_inv<true> : k_fft_x_inv<false>, n[4], kThreadsX, pa[4].smem, kCarveout, st, gk, c->g4, c->fft_twid, pa[4].blocks, c->d_sys, c->D, c->fft_points, c->field_layout, ahead, off[4]);
+  if (c->fft_plane)
+    tild_launch_early(n[4] <= 296 ? k_fft_plane_inv<512> : k_fft_plane_inv<256>, n[4], n[4] <= 296 ? 512 : 256, pa[4].smem, kCarveout, st, gk, c->g4, c->kd, c->fft_twid, pa[4].blocks,
+                      c->d_sys, c->field_layout, ahead, off[4]);
+  else
+    tild_launch_early(dir[0] ? k_fft_x_inv<true> : k_fft_x_inv<false>, n[4], kThreadsX, pa[4].smem, kCarveout, st, gk, c->g4, c->fft_twid, pa[4].blocks, c->d_sys, c->D, c->fft_points, c->field_layout, ahead, off[4]);
   c->launches += 2;
   return tild_check(c, cudaGetLastError(), "grid passes");
 }

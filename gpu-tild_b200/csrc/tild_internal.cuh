@@ -172,6 +172,7 @@ struct tild_ctx {
   float2* fft_twid = nullptr;
   float* ztab = nullptr;                 // multipliers in the z pass's order
   bool fft_direct[3] = {false, false, false};  // of some shape
+  bool fft_plane = false;                // x and y passes of whole planes
   bool fft_wide = false;                 // 16 columns per CTA in the y inverse pass
   int fft_points = 1024;                 // points per field of an x pass's CTA
   // The next integrating step is the last of its call: it stores the float densities (only they can be
