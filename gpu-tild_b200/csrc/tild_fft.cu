@@ -903,6 +903,7 @@ __host__ __device__ inline int plane_exchange(int nx, int ny, int r1x, int r2x) 
   return rows > nx * ny ? rows : nx * ny;
 }
 
+template <bool DIRECT>
 __global__ void __launch_bounds__(kThreadsPlane, 1024 / kThreadsPlane)
     k_fft_plane_fwd(unsigned long long* __restrict__ fx, float* __restrict__ rho, float2* __restrict__ zk,
                     const float2* __restrict__ twid, const int2* __restrict__ blocks, const SysDev* __restrict__ sysd,
@@ -913,7 +914,7 @@ __global__ void __launch_bounds__(kThreadsPlane, 1024 / kThreadsPlane)
   const Lines g(sd.g, 3);
   const int nx = g.nx, ny = g.ny, npt = nx * ny;
   const int R1 = sd.fft_r1[0], R2 = sd.fft_r2[0], R2p = R2 | 1, Y1 = sd.fft_r1[1], Y2 = sd.fft_r2[1];
-  const float2 *twr = twid + sd.fft_tw[0] + sd.fft_twr, *twy = twid + sd.fft_tw[1];
+  const float2 *tw = twid + sd.fft_tw[0], *twr = tw + sd.fft_twr, *twy = twid + sd.fft_tw[1];
   const int p = bk.y / g.nz, plane = bk.y - p * g.nz;
   const bool two = 2 * p + 1 < sd.T + sd.C, paired = sd.fwd_packed;
   float2* in = ex + plane_exchange(nx, ny, R1, R2);
@@ -971,7 +972,7 @@ __global__ void __launch_bounds__(kThreadsPlane, 1024 / kThreadsPlane)
     }
   });
   __syncthreads();
-  second_stage<false>(threadIdx.x, kThreadsPlane, ny * R1, R1, R2, 1, twr, [&](int q) { return ex + q * R2p; },
+  second_stage<DIRECT>(threadIdx.x, kThreadsPlane, ny * R1, R1, R2, 1, tw, [&](int q) { return ex + q * R2p; },
                       [&](int q) {
                         const int line = dk.div(q);
                         return in + line * nx + (q - line * R1);
@@ -996,7 +997,7 @@ __global__ void __launch_bounds__(kThreadsPlane, 1024 / kThreadsPlane)
   __syncthreads();
   float2* z = zk + sd.zk0 + (long long)p * g.M + (long long)plane * npt;
   const unsigned step = Y1 * nx * sizeof(float2);
-  second_stage<false>(threadIdx.x, kThreadsPlane, nx * Y1, Y1, Y2, Y1 * nx, twy, [&](int q) { return ex + q; },
+  second_stage<DIRECT>(threadIdx.x, kThreadsPlane, nx * Y1, Y1, Y2, Y1 * nx, twy, [&](int q) { return ex + q; },
                       [&](int q) { return Run(z + q, step); }, [](const Run& d, int k2, float2 v) { d[k2] = v; });
 }
 
@@ -1008,7 +1009,7 @@ struct NodeRun {
   float *a, *b;
   int x;
 };
-template <int THREADS>
+template <int THREADS, bool DIRECT>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
     k_fft_plane_inv(const float2* __restrict__ gk, float4* __restrict__ g4_all, const float* __restrict__ kd_all,
                     const float2* __restrict__ twid, const int2* __restrict__ blocks, const SysDev* __restrict__ sysd,
@@ -1019,7 +1020,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
   const Lines g(sd.g, 3);
   const int nx = g.nx, ny = g.ny, npt = nx * ny;
   const int R1 = sd.fft_r1[0], R2 = sd.fft_r2[0], R2p = R2 | 1, Y1 = sd.fft_r1[1], Y2 = sd.fft_r2[1];
-  const float2 *twr = twid + sd.fft_tw[0] + sd.fft_twr, *twy = twid + sd.fft_tw[1];
+  const float2 *tw = twid + sd.fft_tw[0], *twr = tw + sd.fft_twr, *twy = twid + sd.fft_tw[1];
   const int f = bk.y % 3, r = bk.y / 3, p = r / g.nz, plane = r - p * g.nz;  // f: x, y, z derivative
   float2* pl = ex + plane_exchange(nx, ny, R1, R2);
   const float2* src = gk + sd.gkp0 + (long long)p * 3 * g.M + (f == 2 ? 2 * g.M : 0) + (long long)plane * npt;
@@ -1052,7 +1053,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
     }
   });
   __syncthreads();
-  second_stage<false>(threadIdx.x, THREADS, nx * Y1, Y1, Y2, Y1 * nx, twy, [&](int q) { return ex + q; },
+  second_stage<DIRECT>(threadIdx.x, THREADS, nx * Y1, Y1, Y2, Y1 * nx, twy, [&](int q) { return ex + q; },
                       [&](int q) { return PlaneValue{pl + q, f ? 0.f : __ldg(kx + (q - dx.div(q) * nx))}; },
                       [&](const PlaneValue& d, int k2, float2 v) {
                         d.p[k2 * (Y1 * nx)] = f ? v : make_float2(-d.k * v.y, d.k * v.x);
@@ -1078,7 +1079,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
   const bool two = 2 * p + 1 < sd.T + sd.C, linear = layout == TILD_FIELD_LINEAR;
   const long long second = 4 * sd.Mb;
   const int zoff = linear ? plane * npt : tild_field_off(layout, 2, plane, sd.g);
-  second_stage<false>(threadIdx.x, THREADS, ny * R1, R1, R2, 1, twr, [&](int q) { return ex + q * R2p; },
+  second_stage<DIRECT>(threadIdx.x, THREADS, ny * R1, R1, R2, 1, tw, [&](int q) { return ex + q * R2p; },
                       [&](int q) {
                         const int line = dk.div(q), row = zoff + (linear ? line * nx : tild_field_off(layout, 1, line, sd.g));
                         float* at = ga + 4ll * row;
@@ -1187,14 +1188,9 @@ int tild_fft_setup(tild_ctx* c) {
     for (int s : b.systems)
       if (b.own) points += (c->sys[s].T + c->sys[s].C + 1) / 2 * c->sys[s].g.M;
   c->fft_points = (int)std::min(1024ll, std::max(256ll, points / 592));
-  // small planes without direct transforms in x or y
   c->fft_plane = D == 3;
-  for (const Bucket& b : c->buckets) {
-    int r1, r2;
-    if (!b.own) continue;
-    c->fft_plane = c->fft_plane && b.nx[0] * b.nx[1] <= kPlanePoints;
-    for (int a = 0; a < 2 && c->fft_plane; a++) c->fft_plane = split_length(b.nx[a], &r1, &r2) && r2 <= 16;
-  }
+  for (const Bucket& b : c->buckets)
+    if (b.own) c->fft_plane = c->fft_plane && b.nx[0] * b.nx[1] <= kPlanePoints;
   c->fft_wide = points >= 16 * 32 * 592;  // the y inverse pass still has some CTAs of 16 columns for every SM
   std::vector<int2> tab[5];
   long long ztotal = 0;
@@ -1276,7 +1272,9 @@ int tild_fft_setup(tild_ctx* c) {
       return TILD_ERR_CUDA;
   }
   auto both = [](auto* regular, auto* direct) { return allow_smem(regular) && allow_smem(direct); };
-  const bool okattr = allow_smem(k_fft_plane_fwd) && both(k_fft_plane_inv<256>, k_fft_plane_inv<512>) && allow_smem(k_fft_x_fwd) && both(k_fft_y_fwd<false>, k_fft_y_fwd<true>) &&
+  const bool okattr = both(k_fft_plane_fwd<false>, k_fft_plane_fwd<true>) &&
+                      both(k_fft_plane_inv<256, false>, k_fft_plane_inv<256, true>) &&
+                      both(k_fft_plane_inv<512, false>, k_fft_plane_inv<512, true>) && allow_smem(k_fft_x_fwd) && both(k_fft_y_fwd<false>, k_fft_y_fwd<true>) &&
                       both(k_fft_z_kmul<false>, k_fft_z_kmul<true>) && both(k_fft_y_inv<8, false>, k_fft_y_inv<8, true>) &&
                       both(k_fft_y_inv<16, false>, k_fft_y_inv<16, true>) && both(k_fft_x_inv<false>, k_fft_x_inv<true>);
   if (!okattr) {
@@ -1332,7 +1330,7 @@ int tild_fft_run(tild_ctx* c, const Bucket* b, bool integrate, bool active, cuda
   const bool* dir = b ? b->fft_direct : c->fft_direct;
   if (!b) tild_mark(c, STAGE_ZERO);
   if (c->fft_plane)
-    tild_launch_early(k_fft_plane_fwd, n[0], kThreadsPlane, pa[0].smem, kCarveout, st, c->rho_fx, c->rho, zk, c->fft_twid, pa[0].blocks,
+    tild_launch_early(dir[0] || dir[1] ? k_fft_plane_fwd<true> : k_fft_plane_fwd<false>, n[0], kThreadsPlane, pa[0].smem, kCarveout, st, c->rho_fx, c->rho, zk, c->fft_twid, pa[0].blocks,
                       c->d_sys, wr, ahead, off[0]);
   else
     tild_launch_early(k_fft_x_fwd, n[0], kThreads, pa[0].smem, kCarveout, st, c->rho_fx, c->rho, zk, c->fft_twid, pa[0].blocks, c->d_sys, c->D, c->fft_points, wr, ahead, off[0]);
@@ -1357,7 +1355,9 @@ int tild_fft_run(tild_ctx* c, const Bucket* b, bool integrate, bool active, cuda
   }
   if (!b) tild_mark(c, STAGE_INTERLEAVE);
   if (c->fft_plane)
-    tild_launch_early(n[4] <= 296 ? k_fft_plane_inv<512> : k_fft_plane_inv<256>, n[4], n[4] <= 296 ? 512 : 256, pa[4].smem, kCarveout, st, gk, c->g4, c->kd, c->fft_twid, pa[4].blocks,
+    tild_launch_early(dir[0] || dir[1] ? (n[4] <= 296 ? k_fft_plane_inv<512, true> : k_fft_plane_inv<256, true>)
+                                       : (n[4] <= 296 ? k_fft_plane_inv<512, false> : k_fft_plane_inv<256, false>),
+                      n[4], n[4] <= 296 ? 512 : 256, pa[4].smem, kCarveout, st, gk, c->g4, c->kd, c->fft_twid, pa[4].blocks,
                       c->d_sys, c->field_layout, ahead, off[4]);
   else
     tild_launch_early(dir[0] ? k_fft_x_inv<true> : k_fft_x_inv<false>, n[4], kThreadsX, pa[4].smem, kCarveout, st, gk, c->g4, c->fft_twid, pa[4].blocks, c->d_sys, c->D, c->fft_points, c->field_layout, ahead, off[4]);
