@@ -1093,7 +1093,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 }
 
 // fieldphase on the interleaved field: type a gets +rho_a f_r, type b -rho_b f_r (planar densities)
-__global__ void k_fieldphase_nodes(float4* __restrict__ g4, long long Mb, const float* __restrict__ rho,
+__global__ void k_fieldphase_nodes(float4* g4, long long Mb, const float* rho,
                                    const float* __restrict__ fr, int a, int b, Geom g, int D, int layout) {
   const long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (m >= g.M) return;
@@ -1104,6 +1104,10 @@ __global__ void k_fieldphase_nodes(float4* __restrict__ g4, long long Mb, const 
     dst = tild_field_off(layout, 0, x, g) + tild_field_off(layout, 1, y, g) + tild_field_off(layout, 2, z, g);
   }
   const float f[3] = {fr[m], fr[g.M + m], D == 3 ? fr[2 * g.M + m] : 0.f};
+  grid_launch_next();
+  grid_wait();
+  g4 = after_wait(g4);
+  rho = after_wait(rho);
   const float ra = rho[(long long)a * g.M + m], rb = rho[(long long)b * g.M + m];
   float4 v = g4[(long long)a * Mb + dst];
   v.x += ra * f[0];
@@ -1367,8 +1371,8 @@ int tild_fft_run(tild_ctx* c, const Bucket* b, bool integrate, bool active, cuda
 
 int tild_fieldphase_nodes(tild_ctx* c, const FieldK& fk) {
   const SysHost& h = c->sys[fk.sys];
-  k_fieldphase_nodes<<<nblk(h.g.M, 256), 256, 0, c->stream>>>(c->g4 + h.g4_0, h.Mb, c->rho + h.grid0, c->frfield + fk.fr0,
-                                                               fk.a, fk.b, h.g, h.D, c->field_layout);
+  tild_launch_early(k_fieldphase_nodes, (int)nblk(h.g.M, 256), 256, 0, kCarveout, c->stream, c->g4 + h.g4_0, h.Mb, c->rho + h.grid0,
+                    c->frfield + fk.fr0, fk.a, fk.b, h.g, h.D, c->field_layout);
   c->launches++;
   return tild_check(c, cudaGetLastError(), "fieldphase");
 }
