@@ -173,7 +173,7 @@ def ensemble_bytes(systems) -> dict:
     """Algorithmic bytes of one launch of each stage over all systems, and of one whole step."""
     tot = collections.Counter()
     for s in systems:
-        tot.update(stage_bytes(s))
+        tot.update(stage_bytes(s, passes=False))
         tot["step"] += step_bytes(s)
     return dict(tot)
 
@@ -285,8 +285,10 @@ def make_system(workload: str):
 # ------------------------------------------------------------------------------------------
 # algorithmic bytes per launch of each stage (the roofline numerators)
 # ------------------------------------------------------------------------------------------
-def stage_bytes(s) -> dict:
-    """Compulsory HBM bytes of one launch of each stage's kernel, each array touched once."""
+def stage_bytes(s, passes: bool = True) -> dict:
+    """Compulsory HBM bytes of one launch of each stage's kernel, each array touched once.  passes: the
+    grid stages are the library's own passes (single systems and slot batches) and their names stand for
+    x forward, y forward, z with the multiply, y inverse and x inverse; else library transforms."""
     ns, D, T = s.ns, s.dim, s.ntypes
     C = 1 if s.charges is not None else 0
     M = int(np.prod(s.nx[:D]))
@@ -296,15 +298,25 @@ def stage_bytes(s) -> dict:
     # x_n (16), bead id, bond info, partners (4 + 4 + 12), x_{n-1} read and x_{n+1} write (32),
     # GJF noise read and write (24), charge (4)
     per_bead_gather = 16 + 20 + 32 + (24 if gjf else 0) + 4 * C
-    return {
-        "sort": 0,
+    pts = 4 * ((T + C + 1) // 2) * 2 * M                   # one complex field of every channel pair
+    grid = {
+        "fix2float": (T + C) * M * 16 + pts,               # read and clear u64, write the pair spectra
+        "r2c": 2 * pts if D == 3 else 0,
+        "kmul": 3 * pts + (T * (T + 1) // 2 + C) * Mh * 4,
+        "c2r": 5 * pts if D == 3 else 0,
+        "interleave": D * pts + (T + C) * M * 16,
+    } if passes else {
         "fix2float": (T + C) * M * (8 + 4 + 8),            # read u64, write f32, clear u64
-        "spread": ns * (16 + 4 * C) + (T + C) * M * 16,     # positions; u64 accumulator RMW
         "r2c": (T + C) * (M * 4 + Mh * 8),
         "kmul": (T + C) * Mh * 8 + nfft * Mh * 4 + C * Mh * 4 + (T + C) * D * Mh * 8,
         "c2r": (T + C) * D * (Mh * 8 + M * 4),
-        "fieldphase": 0,
         "interleave": (T + C) * M * (D * 4 + 16),
+    }
+    return {
+        "sort": 0,
+        **grid,
+        "spread": ns * (16 + 4 * C) + (T + C) * M * 16,     # positions; u64 accumulator RMW
+        "fieldphase": 0,
         "gather": ns * per_bead_gather + (T + C) * M * 16,  # every float4 field node read once
         "step_tail": 0,
     }

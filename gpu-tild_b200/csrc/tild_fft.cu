@@ -4,8 +4,10 @@
 //   x forward    u64 accumulator -> float densities (kept for density reads) -> x transform
 //   y forward    in place                                                        (3D)
 //   z            z transform, k-space multiply, and the inverse z transforms of P and -i kz P
-//   y inverse    P -> P and -i ky P, and the z derivative                        (3D)
-//   x inverse    three fields at once, -i kx on the first, written as float4 nodes
+//   y inverse    P -> -i kx P and -i ky P, and the z derivative                  (3D)
+//   x inverse    three fields at once, written as float4 nodes
+//
+// (small planes take x and y in one kernel each way).
 //
 // The channels (types, then the charge grid) are transformed in pairs, channel 2p as the real and
 // 2p + 1 as the imaginary part of one complex field (an odd last channel with a zero partner).

@@ -1,5 +1,6 @@
-// tild_step.cu — the per-step hot path over all systems of an engine: spread -> batched R2C ->
-// k-space multiply -> batched C2R -> fused gather + bonds + integrators.
+// tild_step.cu — the per-step hot path over all systems of an engine: spread -> grid passes
+// (tild_fft.cu; plain batches and other grid shapes: conversion -> batched R2C -> k-space multiply ->
+// batched C2R -> interleave) -> fused gather + bonds + integrators.
 //
 // Replaces forces() (forces.cu:42-196) followed by Integrator::Integrate_2()
 // (integrator.cu:24-39).  Differences of formulation, each exact in real arithmetic:

@@ -120,3 +120,21 @@ def test_stencil_divisions_are_correctly_rounded(order):
         assert np.array_equal(inds[:, k], i[0] + (i[1] + i[2] * nx[1]) * nx[0])
         assert np.array_equal(w[:, k], W[0][a[0]] * W[1][a[1]] * W[2][a[2]] / gvol)
         k += 1
+
+
+def test_slot_batch_mixes_passes_and_library_shapes():
+    """Shapes that take the passes, shapes that do not, and an inactive system, in one slot batch."""
+    systems = [_system(nx, seed=k) for k, nx in enumerate([(16, 18, 20), (12, 125, 10), (60, 9, 50), (29, 12, 10)])]
+    with tild.Batch(systems, capacity=[s.ns + 300 for s in systems]) as B:
+        fb = [B.forces(i) for i in range(len(systems))]
+        B.set_active(2, False)
+        x2 = B.get_state(2)[0]
+        B.step(19)
+        assert np.array_equal(x2, B.get_state(2)[0])
+        rho = [B.density(i) for i in range(len(systems))]
+        upe = [B.observables(i)["upe"] for i in range(len(systems))]
+    for i, s in enumerate(systems):
+        assert rel_l2(fb[i], oracle.Oracle(s).forces(s.x, 0)) < FORCE_RTOL, i
+        counts = np.bincount(s.types, minlength=2)
+        assert np.allclose(rho[i].astype(np.float64).sum(1) * 0.125, counts, rtol=1e-5)
+        assert np.isfinite(upe[i])
