@@ -1169,9 +1169,9 @@ bool allow_smem(K* k) {
 
 // Whether a grid shape takes these passes.  Measured against the library transforms with their separate
 // conversion, multiply and interleave kernels, us a step of a small diblock system, here / library:
-// 64^3 39.4 / 44.3, 96^3 69.8 / 94.4, 128^3 121 / 147, 94^3 (2 x 47) 122 / 235.  Prime edges, which take
-// the direct transform, are about even (29^3 42.3 / 40.0, 61^3 74.2 / 77.1, 113^3 382 / 448), and 8 slots
-// of 24^3 to 45^3 are 62 / 111.  A second factor above 16 that is not prime (125 = 5 x 25: 213 / 164) and a
+// 40^3 25.8 / 38.7, 64^3 36.4 / 44.6, 96^3 62.8 / 95.7, 128^3 117 / 147, 256^3 844 / 1039, 94^3 (2 x 47)
+// 131 / 235.  Prime edges, which take the direct transform: 29^3 31.1 / 37.8, 61^3 75.8 / 76.7, 113^3
+// 401 / 448; 8 slots of 24^3 to 45^3 59 / 111.  A second factor above 16 that is not prime (125 = 5 x 25: 213 / 164) and a
 // 2D grid whose second axis is prime (101^2, 7 CTAs in the z pass: 49.6 / 36.3) stay with the library.
 bool tild_fft_supports(const int* nx, int D, int T, int C) {
   int a, b;
