@@ -796,6 +796,7 @@ bool all_ready(tild_ctx* c) {
 // Host bookkeeping of `n` integrating steps that ran inside a graph replay (the device side,
 // including step counters and buffer rotations, is in the graph).
 void account_replayed_steps(tild_ctx* c, int n, long long launches, int nsorts) {
+  tild_spectra_stale(c);
   for (int s = 0; s < c->nsys; s++) {
     SysHost& h = c->sys[s];
     if (!h.active) continue;

@@ -137,6 +137,7 @@ struct Bucket {     // systems sharing one grid shape: one batched R2C plan and 
   // own grid passes (tild_fft.cu): the forward cuFFT plan serves the observables' spectra only
   bool own = false;
   bool spectra = false;                  // rhok holds the library spectra of the last force evaluation
+                                         // (tild_spectra_stale)
   int fft_blk0[5] = {0}, fft_nblk[5] = {0};
   bool fft_direct[3] = {false, false, false};  // the x, y, z axis takes the direct transform
   int cta_spec0 = 0, n_cta_spec = 0;     // the shape's range of spectrum blocks (k-space multiply)
@@ -531,6 +532,11 @@ int tild_fft_setup(tild_ctx* c);
 void tild_fft_free(tild_ctx* c);
 int tild_fft_run(tild_ctx* c, const Bucket* b, bool integrate, bool active, cudaStream_t st);
 int tild_fieldphase_nodes(tild_ctx* c, const FieldK& fk);
+// A force evaluation was launched, by itself or inside a replayed graph: the own passes leave their
+// partly transformed fields in rhok, the library transforms their spectra.
+inline void tild_spectra_stale(tild_ctx* c) {
+  for (Bucket& b : c->buckets) b.spectra = !b.own;
+}
 int tild_obs_compute(tild_ctx* c, int s, tild_obs* o); // tild_obs.cu
 int tild_sk_acc_run(tild_ctx* c, int s, int slot, int type);
 int tild_table_scratch(tild_ctx* c);

@@ -1494,7 +1494,7 @@ int tild_run_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys) {
     }
     c->evals_since_sort++;
   }
-  for (Bucket& b : c->buckets) b.spectra = !b.own;  // own passes keep no spectra
+  tild_spectra_stale(c);
   const std::vector<char> on = integrate ? tild_buckets_on(c) : std::vector<char>(c->buckets.size(), 1);
   if (c->fft_pipeline >= 2 && c->lanes > 0 && c->fields.empty()) {
     // each grid shape runs its whole step in order on its stream: spread, conversion, R2C,
