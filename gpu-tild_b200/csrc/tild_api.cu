@@ -796,7 +796,7 @@ bool all_ready(tild_ctx* c) {
 // Host bookkeeping of `n` integrating steps that ran inside a graph replay (the device side,
 // including step counters and buffer rotations, is in the graph).
 void account_replayed_steps(tild_ctx* c, int n, long long launches, int nsorts) {
-  tild_spectra_stale(c);
+  tild_spectra_stale(c, tild_buckets_on(c));
   for (int s = 0; s < c->nsys; s++) {
     SysHost& h = c->sys[s];
     if (!h.active) continue;
@@ -820,6 +820,7 @@ constexpr int kMinGraphSteps = 8;  // shorter runs launch directly
 // run as direct launches.
 int run_steps(tild_ctx* c, int n) {
   const int len = c->sort_interval > 0 ? 2 * c->sort_interval : c->graph_len;
+  if (n > 0 && tild_keep_spectra(c)) return TILD_ERR_CUDA;
   while (n > 0) {
     const bool aligned = c->sort_interval <= 0 || c->steps_since_sort >= c->sort_interval;
     int L = 0;
@@ -1566,8 +1567,8 @@ int32_t tild_profile_steps(tild_ctx* c, int32_t nsteps, double* stage_ms, int32_
   cudaSetDevice(c->device);
   c->prof_ev.clear();
   c->prof_stage.clear();
+  int rc = tild_keep_spectra(c);
   c->profiling = true;
-  int rc = TILD_OK;
   for (int k = 0; k < nsteps && !rc; k++) rc = tild_run_forces(c, true, nullptr, -1);
   c->profiling = false;
   cudaEvent_t last;

@@ -532,11 +532,13 @@ int tild_fft_setup(tild_ctx* c);
 void tild_fft_free(tild_ctx* c);
 int tild_fft_run(tild_ctx* c, const Bucket* b, bool integrate, bool active, cudaStream_t st);
 int tild_fieldphase_nodes(tild_ctx* c, const FieldK& fk);
-// A force evaluation was launched, by itself or inside a replayed graph: the own passes leave their
-// partly transformed fields in rhok, the library transforms their spectra.
-inline void tild_spectra_stale(tild_ctx* c) {
-  for (Bucket& b : c->buckets) b.spectra = !b.own;
+// A force evaluation of the shapes in `on` was launched, by itself or inside a replayed graph: the own
+// passes leave their partly transformed fields in rhok, the library transforms their spectra.
+inline void tild_spectra_stale(tild_ctx* c, const std::vector<char>& on) {
+  for (size_t k = 0; k < on.size(); k++)
+    if (on[k]) c->buckets[k].spectra = !c->buckets[k].own;
 }
+int tild_keep_spectra(tild_ctx* c);                                    // tild_step.cu
 int tild_obs_compute(tild_ctx* c, int s, tild_obs* o); // tild_obs.cu
 int tild_sk_acc_run(tild_ctx* c, int s, int slot, int type);
 int tild_table_scratch(tild_ctx* c);

@@ -1494,8 +1494,8 @@ int tild_run_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys) {
     }
     c->evals_since_sort++;
   }
-  tild_spectra_stale(c);
   const std::vector<char> on = integrate ? tild_buckets_on(c) : std::vector<char>(c->buckets.size(), 1);
+  tild_spectra_stale(c, on);
   if (c->fft_pipeline >= 2 && c->lanes > 0 && c->fields.empty()) {
     // each grid shape runs its whole step in order on its stream: spread, conversion, R2C,
     // k-space multiply, C2R, interleave and gather, so one shape's transforms overlap another's
@@ -1691,6 +1691,22 @@ int tild_density_planar(tild_ctx* c, int s, float* dst, cudaStream_t st) {
   }
   return tild_check(c, cudaMemcpyAsync(dst, c->rho + h.grid0, sizeof(float) * (size_t)(h.T + h.C) * M,
                                        cudaMemcpyDeviceToDevice, st), "copy densities") ? TILD_ERR_CUDA : TILD_OK;
+}
+
+// Steps without a moving system of a shape leave its spectra as the last evaluation made them, while its
+// densities follow the held positions: before such steps the spectra are taken from the densities that the
+// evaluation stored.
+int tild_keep_spectra(tild_ctx* c) {
+  const std::vector<char> on = tild_buckets_on(c);
+  for (size_t k = 0; k < on.size(); k++) {
+    Bucket& b = c->buckets[k];
+    bool evaluated = false;
+    for (int s : b.systems) evaluated = evaluated || c->sys[s].have_forces;
+    if (on[k] || b.spectra || !evaluated) continue;
+    if (exec_forward(c, b)) return TILD_ERR_CUDA;
+    b.spectra = true;
+  }
+  return TILD_OK;
 }
 
 // A system's density half spectra in the R2C layout [(T + C)][Mh], valid after its last force

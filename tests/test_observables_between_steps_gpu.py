@@ -68,3 +68,32 @@ def test_slot_batch_records_after_replayed_graphs():
                 assert oa["upe"] == ob["upe"] and np.array_equal(oa["ptens"], ob["ptens"]), i
         for i in range(3):
             assert np.array_equal(A.sk_get(i, 0)[0], B.sk_get(i, 0)[0]), i
+
+
+@pytest.mark.parametrize("read_between", [False, True])
+@pytest.mark.parametrize("steps", [5, 64])
+def test_a_shape_at_rest_keeps_its_record(steps, read_between):
+    """A system whose whole shape takes no part in the steps keeps the energies, virials and S(k) of its
+    last force evaluation, read before or not."""
+    systems = [small_diblock(3, 1, seed=3), charged_system()]
+    with tild.Batch(systems, capacity=[s.ns + 100 for s in systems]) as B:
+        B.step(10)
+        want = B.observables(1)
+        B.sk_accumulate(1, 0, 0)
+        sk = B.sk_get(1, 0)[0]
+    with tild.Batch(systems, capacity=[s.ns + 100 for s in systems]) as B:
+        B.step(10)
+        if read_between:
+            B.observables(1)
+        B.set_active(1, False)
+        for _ in range(3):
+            B.step(steps)
+            got = B.observables(1)
+            assert got["upe"] - got["ubond"] == pytest.approx(want["upe"] - want["ubond"], rel=1e-12)
+            assert np.array_equal(got["style_virial"], want["style_virial"])
+        B.sk_accumulate(1, 0, 0)
+        assert np.array_equal(B.sk_get(1, 0)[0], sk)
+        B.set_active(1, True)       # and moves on from there
+        B.step(steps)
+        moved = B.observables(1)
+    assert moved["upe"] != want["upe"]
