@@ -91,10 +91,10 @@ struct SysDev {
   float bond_k[TILD_MAX_BOND_TYPES], bond_req[TILD_MAX_BOND_TYPES];
 };
 
-// A system's state `ahead` steps after the device counters were last advanced: whether it still moves,
-// and its completed steps.
+// Whether a system still moves `ahead` steps after the device counters were last advanced.  One that is
+// active there takes that step whatever its stop, and leaves the active set after it.
 __device__ __forceinline__ bool active_at(const SysDev& sd, int ahead) {
-  return sd.active && (sd.stop_at < 0 || sd.step + ahead < sd.stop_at);
+  return sd.active && (ahead == 0 || sd.stop_at < 0 || sd.step + ahead < sd.stop_at);
 }
 
 struct FieldK {     // one fieldphase style

@@ -1196,9 +1196,10 @@ __global__ void __launch_bounds__(256, (P >= 4 ? 2 : 3)) k_gather_box(
 __global__ void k_advance_steps(SysDev* __restrict__ sysd, int nsys, int n) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsys || !sysd[s].active) return;
-  const long long stop = sysd[s].stop_at, step = sysd[s].step + n;
-  sysd[s].step = stop >= 0 && step > stop ? stop : step;
-  if (stop >= 0 && step >= stop) sysd[s].active = 0;
+  const long long stop = sysd[s].stop_at, step = sysd[s].step;
+  const long long moved = stop < 0 || step + n < stop ? n : max(stop - step, 1ll);  // as active_at counts them
+  sysd[s].step = step + moved;
+  if (stop >= 0 && step + moved >= stop) sysd[s].active = 0;
 }
 
 // Order <= 1 always spreads directly; order >= 2 uses the shared box unless the tuner chose the

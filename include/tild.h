@@ -268,7 +268,8 @@ int32_t tild_batch_capacity(tild_batch* b, int32_t sys, int32_t* capacity);
 int32_t tild_batch_load(tild_batch* b, int32_t sys, const tild_config* cfg);
 /* System `sys` leaves the active set on the device when its step counter reaches stop_at
  * (-1: never), so a stepping call may run past a system's last step: that system takes exactly
- * stop_at - step steps.  Step counters and activity are read back after every stepping call. */
+ * stop_at - step steps (one step when it is active at or past stop_at already).  Step counters and
+ * activity are read back after every stepping call. */
 int32_t tild_batch_set_stop(tild_batch* b, int32_t sys, int64_t stop_at);
 int32_t tild_batch_get_active(tild_batch* b, int32_t sys, int32_t* active);
 
