@@ -438,6 +438,13 @@ __device__ __forceinline__ void spline_w(float gdx, float H, float rH, float* W)
   }
 }
 
+// Positions so far out that x / dx overflows make div_by's corrections NaN, which would count as index 0:
+// they are out of range, and x itself says on which side.
+__device__ __forceinline__ int cell_of(float x, float dx, float rdx) {
+  const float q = div_by(x, dx, rdx);
+  return (int)(q == q ? q : x);
+}
+
 // Grid index of one bead along one axis (device_grid_utils.cu:256-266): even orders use the
 // nearest node, odd orders the containing cell; returns the first stencil node and sets gdx, the
 // offset from that node or cell centre that the spline weights take.
@@ -445,10 +452,10 @@ template <int P>
 __device__ __forceinline__ int axis_index(float xj, float dxj, float rdx, float& gdx) {
   int gi;
   if (P % 2 == 0) {
-    gi = (int)div_by(xj + 0.5f * dxj, dxj, rdx);
+    gi = cell_of(xj + 0.5f * dxj, dxj, rdx);
     gdx = xj - (float)gi * dxj;
   } else {
-    gi = (int)div_by(xj, dxj, rdx);
+    gi = cell_of(xj, dxj, rdx);
     gdx = xj - ((float)gi + 0.5f) * dxj;
   }
   return gi - P / 2;
