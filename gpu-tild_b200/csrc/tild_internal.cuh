@@ -93,8 +93,11 @@ struct SysDev {
 
 // Whether a system still moves `ahead` steps after the device counters were last advanced.  One that is
 // active there takes that step whatever its stop, and leaves the active set after it.
+__device__ __forceinline__ bool active_at(int active, long long step, long long stop_at, int ahead) {
+  return active && (ahead == 0 || stop_at < 0 || step + ahead < stop_at);
+}
 __device__ __forceinline__ bool active_at(const SysDev& sd, int ahead) {
-  return sd.active && (ahead == 0 || sd.stop_at < 0 || sd.step + ahead < sd.stop_at);
+  return active_at(sd.active, sd.step, sd.stop_at, ahead);
 }
 
 struct FieldK {     // one fieldphase style
@@ -335,7 +338,10 @@ inline void tild_mark(tild_ctx* c, int stage) {
 // A kernel launched with tild_launch_early may start while the kernel before it in the stream still
 // runs, once all CTAs of that kernel have called grid_launch_next() or ended.  It touches what earlier
 // kernels write or still read only after grid_wait(), through pointers passed through after_wait()
-// (the compiler may move read-only loads across the wait otherwise).
+// (the compiler may move read-only loads across the wait otherwise).  Every CTA waits before it ends, since
+// the next kernel takes this one's end for that of all before it.
+// One exception: the early gather reads what the particle kernels of earlier steps left (their positions,
+// noise, topology and step counters) before its wait, with load_done().
 __device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <class T>
@@ -343,6 +349,39 @@ __device__ __forceinline__ T* after_wait(T* p) {
   size_t g = __cvta_generic_to_global(p);  // a global address still: generic loads cost the passes 7 %
   asm volatile("" : "+l"(g)::"memory");
   return static_cast<T*>(__cvta_global_to_generic(g));
+}
+// A read, before grid_wait(), of memory last written by a kernel that is known to have ended: a kernel in
+// between has waited for it, which leaves its writes performed, and called grid_launch_next() only after
+// that.  Strong loads at device scope read what was performed before them; a plain one could still find a
+// line of an earlier step in L1.
+__device__ __forceinline__ int load_done(const int* p) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(p)) : "memory");
+  return v;
+}
+__device__ __forceinline__ long long load_done(const long long* p) {
+  long long v;
+  asm volatile("ld.relaxed.gpu.global.s64 %0, [%1];" : "=l"(v) : "l"(__cvta_generic_to_global(p)) : "memory");
+  return v;
+}
+__device__ __forceinline__ float load_done(const float* p) {
+  float v;
+  asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(__cvta_generic_to_global(p)) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 load_done(const float4* p) {
+  float4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(__cvta_generic_to_global(p))
+               : "memory");
+  return v;
+}
+// The load of kernels with early variants: load_done() there, a plain read elsewhere.
+template <bool EARLY, class T>
+__device__ __forceinline__ T load_if_done(const T* __restrict__ p) {
+  if constexpr (EARLY) return load_done(p);
+  else return *p;
 }
 // carveout: per cent of the SM's 228 KB preferred as shared memory (-1: the function's own setting)
 template <class... P, class... A>

@@ -865,9 +865,16 @@ __device__ __forceinline__ void bead_epilogue(int i, const float4& p, int t, flo
 // EARLY (small systems of order <= 1): a launch that leaves SMs with a CTA or two is one chain of
 // latencies, so everything that does not need the field is read and drawn before the stencil (bond
 // partners, x_{n-1}, noise), at the registers of 2 CTAs per SM; and the kernel starts while the grid
-// passes before it end (the z pass lets its successors start only once the last step's kernels are done,
-// so positions and topology may be read before the wait).  us a step: 40^2 film 17.5 -> 16.1, 40^3 with
-// 157 CTAs 30.8 -> 29.8; 235 CTAs of order 4 70.7 -> 72.3 and 860 of order 1 with charges 130 -> 129.
+// passes before it end.  us a step: 40^2 film 17.5 -> 16.1, 40^3 with 157 CTAs 30.8 -> 29.8 (30.5 with all
+// reads behind the wait); 235 CTAs of order 4 70.7 -> 72.3 and 860 of order 1 with charges 130 -> 129.
+//
+// What it reads before its wait (load_done) was last written by an earlier step's gather, a sort, a packing
+// kernel or the counters' kernel.  None of them calls grid_launch_next(), and the gather ends after its own
+// wait.  The first grid pass of this step waits for the one before it, the z pass waits for the first
+// passes, and it calls grid_launch_next() only after that: no kernel behind it, the gather among them, can
+// start before they have ended and their writes are performed.  So these kernels must not start their
+// successors early, nor the z pass before its wait.  A step on several streams starts after a join of them
+// all, and after the library transforms, which are no early launches, the gather does not start early.
 template <int D, int P, bool INTEG, bool XW, bool CH, int SPR, bool EARLY>
 __global__ void __launch_bounds__(256, EARLY ? 2 : (P >= 4 ? 2 : (P >= 3 ? 4 : (P >= 2 ? 3 : 4)))) k_gather(
     const float4* __restrict__ pos_in, float4* __restrict__ pos_io, float* __restrict__ noise,
@@ -880,14 +887,15 @@ __global__ void __launch_bounds__(256, EARLY ? 2 : (P >= 4 ? 2 : (P >= 3 ? 4 : (
   const int s = cta_sys[blockIdx.x + blk_off];
   const SysDev& sd = sysd[s];
   const int i = (blockIdx.x + blk_off) * blockDim.x + threadIdx.x;
-  const float4 p = pos_in[i];
+  const float4 p = load_if_done<EARLY>(pos_in + i);
   const int t = tild_type_of(p.w);
   float x[3] = {p.x, p.y, p.z};
   const bool finite = isfinite(p.x) && isfinite(p.y) && (D == 2 || isfinite(p.z));
   const int C = sd.C;
-  const float q = (CH && C && t != kPadType) ? charge[i] : 0.f;
+  const float q = (CH && C && t != kPadType) ? load_if_done<EARLY>(charge + i) : 0.f;
   bool sp = false;  // x (after the update) is spread ahead
-  if (!active_at(sd, ahead)) {  // one system per CTA: every thread takes this branch together
+  const long long step = load_if_done<EARLY>(&sd.step);
+  if (!active_at(load_if_done<EARLY>(&sd.active), step, sd.stop_at, ahead)) {  // one system per CTA: every thread takes this branch together
     if (EARLY) grid_wait();
     if (INTEG) pos_io[i] = p;  // inactive systems keep x_n through the buffer rotation
     if (SPR == 0) return;
@@ -946,17 +954,17 @@ __global__ void __launch_bounds__(256, EARLY ? 2 : (P >= 4 ? 2 : (P >= 3 ? 4 : (
     float4 pj[3], po = make_float4(0.f, 0.f, 0.f, 0.f);
     float on0[3] = {0.f, 0.f, 0.f}, z0[3] = {0.f, 0.f, 0.f};
     if (EARLY) {
-      info = bond_info[i];
+      info = load_done(bond_info + i);
       nb = info & 3;
-      bid = bead_id[i];
-      po = pos_io[i];
+      bid = load_done(bead_id + i);
+      po = load_done(pos_io + i);
 #pragma unroll
-      for (int d = 0; d < D; d++) on0[d] = noise[3 * (long long)i + d];
+      for (int d = 0; d < D; d++) on0[d] = load_done(noise + 3 * (long long)i + d);
 #pragma unroll
       for (int bb = 0; bb < 3; bb++)
-        if (bb < nb) pj[bb] = pos_in[bond_nbr[3 * i + bb]];
+        if (bb < nb) pj[bb] = load_done(pos_in + load_done(bond_nbr + 3 * i + bb));
       ig0 = __ffs(sd.type_mask[t]) - 1;
-      if (ig0 >= 0) philox_normal3(sd.seed, (uint32_t)bid, sd.step + ahead + 1, (uint32_t)ig0, z0);
+      if (ig0 >= 0) philox_normal3(sd.seed, (uint32_t)bid, step + ahead + 1, (uint32_t)ig0, z0);
     }
     {
       float W[3][P + 1];
@@ -998,10 +1006,9 @@ __global__ void __launch_bounds__(256, EARLY ? 2 : (P >= 4 ? 2 : (P >= 3 ? 4 : (
       sp = isfinite(x[0]) && isfinite(x[1]) && (D == 2 || isfinite(x[2]));
       if (!sp) atomicOr(status, ST_NONFINITE_POS);
     }
-  } else if (SPR == 0) {
-    return;  // padding slot
-  } else if (EARLY) {
-    grid_wait();
+  } else {  // padding slot
+    if (EARLY) grid_wait();
+    if (SPR == 0) return;
   }
   if constexpr (SPR == 1) cta_spread_box<D, P, CH>(sp, x, t, q, sd, rho_fx_all + sd.grid0, spread_cap, status);
   if constexpr (SPR == 2)
