@@ -702,6 +702,7 @@ int sys_set_topology(tild_ctx* c, int s, const int32_t* types, const float* char
   if (tild_check(c, cudaStreamSynchronize(st), "sync topology")) return TILD_ERR_CUDA;
   h.kbits = spread_kbits(h.p, h.D, h.g.gvol, qmax);
   c->h_sys[s].kbits = h.kbits;
+  c->evals_since_sort = tild_ctx::kUnsorted;
   h.topo_set = true;
   h.state_set = false;
   h.have_forces = false;

@@ -257,7 +257,8 @@ struct tild_ctx {
   int sort_cell_bits = 0;
   int sort_interval = 0;                 // 0: never
   int64_t steps_since_sort = 0;
-  int64_t evals_since_sort = 1 << 20;    // force-only evaluations; none sorted yet
+  static constexpr int64_t kUnsorted = 1 << 20;
+  int64_t evals_since_sort = kUnsorted;  // force-only evaluations; kUnsorted: beads in the caller's order
   long long sorts = 0;
   int spread_cap = 0;                    // shared-memory 32-bit words of the tiled spread
 
