@@ -93,11 +93,8 @@ struct SysDev {
 
 // Whether a system still moves `ahead` steps after the device counters were last advanced.  One that is
 // active there takes that step whatever its stop, and leaves the active set after it.
-__device__ __forceinline__ bool active_at(int active, long long step, long long stop_at, int ahead) {
-  return active && (ahead == 0 || stop_at < 0 || step + ahead < stop_at);
-}
 __device__ __forceinline__ bool active_at(const SysDev& sd, int ahead) {
-  return active_at(sd.active, sd.step, sd.stop_at, ahead);
+  return sd.active && (ahead == 0 || sd.stop_at < 0 || sd.step + ahead < sd.stop_at);
 }
 
 struct FieldK {     // one fieldphase style
@@ -377,12 +374,6 @@ __device__ __forceinline__ float4 load_done(const float4* p) {
                : "l"(__cvta_generic_to_global(p))
                : "memory");
   return v;
-}
-// The load of kernels with early variants: load_done() there, a plain read elsewhere.
-template <bool EARLY, class T>
-__device__ __forceinline__ T load_if_done(const T* __restrict__ p) {
-  if constexpr (EARLY) return load_done(p);
-  else return *p;
 }
 // carveout: per cent of the SM's 228 KB preferred as shared memory (-1: the function's own setting)
 template <class... P, class... A>
