@@ -380,17 +380,23 @@ int engine_create(const tild_config* cfgs, int nsys, int device, tild_ctx* c, co
   // shared box costs the gather its L1 share and barriers (both measured on the B200)
   c->spread_ahead = cfgs[0].pmeorder <= 1 ? 1 : 0;
   // Order >= 2 in 3D reads its 27 to 125 field nodes from 4x4x4 bricks: us a step linear / brick, 2.6M
-  // beads on 128^3 order 3 549 / 491, 45^3 order 2 56.5 / 55.8, 90^3 order 4 246 / 235.  Half the shared
-  // box where beads are dense enough that 256 of them stay within it (more CTAs per SM: the same blend
-  // 516 / 491, 45^3 57.6 / 55.8; at 0.45 beads per node and channel most chunks overflow it, 48^3 order 3
-  // 54.3 / 59.4).
+  // beads on 128^3 order 3 549 / 491, 45^3 order 2 56.5 / 55.8, 90^3 order 4 246 / 235.
+  // Half the shared spread box (more CTAs per SM) where 256 beads stay within it, us a step with the whole /
+  // with half: the same blend 516 / 491, 45^3 57.6 / 55.8; on 56^3 order 2 up to 10 types of 0.56 beads per
+  // node each 233 / 224, order 3 4 types of 1.0 169 / 164.  Beyond that chunks overflow it, and at order 3 an
+  // overflowing bead is 64 additions to the global grid: 48^3 with 0.45 per node and channel 54.3 / 59.4, 56^3
+  // 8 types of 0.56 234 / 338, 6 types of 1.6 349 / 354, order 2 12 types of 0.56 278 / 293.  Below 0.75 beads
+  // per node a chunk runs on into the next row of bricks (56^3, one type of 0.56: 54 / 67).
   if (cfgs[0].dim == 3 && cfgs[0].pmeorder >= 2) {
     c->field_layout = TILD_FIELD_BRICK;
-    bool dense = cfgs[0].pmeorder <= 3;
+    const double most = c->P == 2 ? 6144.0 : 4450.0;
+    bool dense = c->P <= 3;
     for (int s = 0; s < nsys; s++) {
       const tild_config& q = cfgs[s];
-      const double nodes = (double)q.nx[0] * q.nx[1] * q.nx[2] * (q.ntypes + (q.do_charges ? 1 : 0));
-      dense = dense && q.ns >= 0.55 * nodes;
+      const int channels = q.ntypes + (q.do_charges ? 1 : 0);
+      const double density = q.ns / ((double)q.nx[0] * q.nx[1] * q.nx[2]);
+      dense = dense && density >= std::max(0.75, 0.55 * channels) &&
+              tild_spread_words(3, c->P, channels, density, kTile) <= most;
     }
     if (dense) c->spread_cap = 6144;
   }

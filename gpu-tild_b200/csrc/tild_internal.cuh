@@ -400,6 +400,15 @@ inline void tild_launch_early(void (*kernel)(P...), int grid, int threads, size_
 // 133 us a step against 139 at 100).
 constexpr int kCarveout = 60;
 
+// Words of the shared box that `beads` sorted beads of a system with `density` beads per node are expected
+// to need: a run of beads / density / 64 bricks along x (2D: of 8x8 tiles), with the stencil's and two nodes
+// of drift's halo, and room for a turn into the next row of bricks (40 %).
+inline double tild_spread_words(int D, int P, int channels, double density, int beads) {
+  const int edge = D == 3 ? 4 : 8, halo = P + 2;
+  const double run = beads / density / 64.0 * edge + halo, side = edge + halo;
+  return 1.4 * channels * run * side * (D == 3 ? side : 1.0);
+}
+
 // ---- small helpers -----------------------------------------------------------------------
 // Per-channel storage of the float4 force field: room for the brick layout (3D: 4x4x4 bricks,
 // edges rounded up to 4), so either layout fits without reallocating.

@@ -1228,24 +1228,17 @@ struct BeadRange {
 };
 inline BeadRange all_beads(tild_ctx* c) { return {c->stream, 0, c->n_cta_bead}; }
 
-// Threads per bead of the box spread.  256 sorted beads cover about V = 256 / density nodes, a run of
-// V / 64 bricks along x; with the stencil's and two nodes of drift's halo their box has to fit the
-// largest shared box with room for a turn into the next row of bricks (40 %), or the chunk adds every
-// node to the global grid: 64^3, 4 channels, 0.49 beads per node, order 3: spread 98 us with 256 beads a
-// CTA, 36 with 64; 90^3 order 4, 0.41: 91 and 70.  Where they fit, fewer beads a CTA clear and flush more
-// words a bead (2.6M blend 126 and 337 us), except in systems that do not fill the SMs (10,000 beads:
-// 10.0 and 7.5 us; 60,000 of order 4: 26 and 20).
+// Threads per bead of the box spread.  The box of 256 sorted beads (tild_spread_words) has to fit the shared
+// one, or the chunk adds every node to the global grid: 64^3, 4 channels, 0.49 beads per node, order 3:
+// spread 98 us with 256 beads a CTA, 36 with 64; 90^3 order 4, 0.41: 91 and 70.  Where they fit, fewer beads
+// a CTA clear and flush more words a bead (2.6M blend 126 and 337 us), except in systems that do not fill
+// the SMs (10,000 beads: 10.0 and 7.5 us; 60,000 of order 4: 26 and 20).
 int spread_share(const tild_ctx* c) {
   if (c->n_cta_bead < 296) return 4;
   int share = 1;
   for (const SysHost& h : c->sys) {
     const double density = (double)h.ns / (double)h.g.M;
-    const int edge = c->D == 3 ? 4 : 8, halo = c->P + 2;
-    auto words = [&](int beads) {
-      const double run = beads / density / 64.0 * edge + halo, side = edge + halo;
-      return 1.4 * (h.T + h.C) * run * side * (c->D == 3 ? side : 1.0);
-    };
-    while (share < 4 && words(256 / share) > 12288.0) share *= 2;
+    while (share < 4 && tild_spread_words(c->D, c->P, h.T + h.C, density, 256 / share) > c->spread_cap) share *= 2;
   }
   return share;
 }
