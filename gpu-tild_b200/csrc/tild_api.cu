@@ -220,11 +220,9 @@ int spread_kbits(int P, int D, double gvol, double qmax) {
 
 }  // namespace
 
-// Spreads the grid-shape buckets over the first `lanes` auxiliary streams (largest first, each to
-// the least loaded stream) and binds their cuFFT plans to them; lanes = 0 keeps every transform on
-// the main stream.
-int tild_assign_lanes(tild_ctx* c, int lanes) {
-  lanes = std::max(0, std::min(lanes, (int)c->aux.size()));
+// Spreads the grid-shape buckets over `lanes` streams: largest first, each to the least loaded one;
+// lanes = 0 keeps all of them on the main stream.
+static void spread_lanes(tild_ctx* c, int lanes) {
   std::vector<int> order(c->buckets.size());
   for (size_t k = 0; k < order.size(); k++) order[k] = (int)k;
   auto work = [&](int k) {
@@ -244,6 +242,14 @@ int tild_assign_lanes(tild_ctx* c, int lanes) {
       b.lane = best;
       load[best] += work(bi);
     }
+  }
+}
+
+// Spreads the buckets over the first `lanes` auxiliary streams and binds their cuFFT plans to them.
+int tild_assign_lanes(tild_ctx* c, int lanes) {
+  lanes = std::max(0, std::min(lanes, (int)c->aux.size()));
+  spread_lanes(c, lanes);
+  for (Bucket& b : c->buckets) {
     if (!b.planned || b.own) continue;  // own passes: the plan serves the observables, on the main stream
     cudaStream_t bs = b.lane >= 0 ? c->aux[b.lane] : c->stream;
     if (tild_check_fft(c, cufftSetStream(b.fwd_packed ? b.c2c_fwd : b.r2c, bs), "plan stream") ||
@@ -500,8 +506,8 @@ int engine_create(const tild_config* cfgs, int nsys, int device, tild_ctx* c, co
     long long pairs = 0;
     // A plain batch keeps the library transforms, whose results its members' long runs then reproduce
     // bit for bit: with the own passes the forces differ by 2e-7 to 4e-7 (relative, as much as either is
-    // from 64 bits), which moved an ensemble's densities by 2e-5 to 4e-5 within 128 steps (296 against
-    // 471 us a step for 40 systems of 24^3 to 48^3).
+    // from 64 bits), which moved an ensemble's densities by 2e-5 to 4e-5 within 128 steps (309 us a step
+    // against 390 with the library, for 40 systems of 24^3 to 48^3 in 25 shapes).
     b.own = nsys == 1 || capacity;
     for (int s : b.systems) b.own = b.own && tild_fft_supports(b.nx, c->D, c->sys[s].T, c->sys[s].C);
     for (int s : b.systems) {
@@ -530,19 +536,29 @@ int engine_create(const tild_config* cfgs, int nsys, int device, tild_ctx* c, co
   c->nbeads = (int)beads;
   // CTA -> system lookup tables (grid and spectrum tables carry each system's first block after them)
   std::vector<int> tb, tspec, tgrid, bspec(nsys), bgrid(nsys);
-  // particle, spectrum and grid blocks in grid-shape order, so each shape's blocks form one range
+  // each shape's particle, spectrum and grid blocks form one range; the spectrum and grid blocks of the
+  // shapes that share a stream (as first assigned) follow one another, so that it takes them in one launch
+  const int naux = c->buckets.size() > 1 ? (int)std::min<size_t>(8, c->buckets.size()) : 0;
+  spread_lanes(c, naux);
   for (Bucket& b : c->buckets) {
     b.cta_bead0 = (int)tb.size();
+    for (int s : b.systems)
+      for (int k = 0; k < c->sys[s].ns_pad / kTile; k++) tb.push_back(s);
+    b.n_cta_bead = (int)tb.size() - b.cta_bead0;
+  }
+  std::vector<int> by_lane(c->buckets.size());
+  for (size_t k = 0; k < by_lane.size(); k++) by_lane[k] = (int)k;
+  std::stable_sort(by_lane.begin(), by_lane.end(), [&](int a, int b) { return c->buckets[a].lane < c->buckets[b].lane; });
+  for (int k : by_lane) {
+    Bucket& b = c->buckets[k];
     b.cta_spec0 = (int)tspec.size();
     b.cta_grid0 = (int)tgrid.size();
     for (int s : b.systems) {
-      for (int k = 0; k < c->sys[s].ns_pad / kTile; k++) tb.push_back(s);
       bspec[s] = (int)tspec.size();
       for (long long k = 0; k < (c->sys[s].g.Mh + 255) / 256; k++) tspec.push_back(s);
       bgrid[s] = (int)tgrid.size();
       for (long long k = 0; k < (c->sys[s].g.M + 255) / 256; k++) tgrid.push_back(s);
     }
-    b.n_cta_bead = (int)tb.size() - b.cta_bead0;
     b.n_cta_spec = (int)tspec.size() - b.cta_spec0;
     b.n_cta_grid = (int)tgrid.size() - b.cta_grid0;
   }
@@ -606,8 +622,7 @@ int engine_create(const tild_config* cfgs, int nsys, int device, tild_ctx* c, co
   if (tild_check(c, cudaStreamSynchronize(st), "init")) return TILD_ERR_CUDA;
   // batched cuFFT plans, one pair per grid shape; with several shapes each plan runs on one of
   // up to 8 auxiliary streams so transforms of different shapes overlap
-  if (c->buckets.size() > 1) {
-    const int naux = (int)std::min<size_t>(8, c->buckets.size());
+  if (naux) {
     c->aux.resize(naux);
     c->ev_join.resize(naux);
     for (int k = 0; k < naux; k++) {
@@ -640,9 +655,11 @@ int engine_create(const tild_config* cfgs, int nsys, int device, tild_ctx* c, co
     b.planned = true;
   }
   if (tild_assign_lanes(c, (int)c->aux.size())) return TILD_ERR_CUDA;
-  // several shapes on the library transforms: each shape's grid stages in sequence on its stream, so that
-  // small transforms overlap other shapes' passes (40 systems of 25 shapes: 411 against 486 us a step
-  // stage by stage; 8 systems of 8 shapes: 107 against 119).  Own passes take all shapes at once.
+  // several shapes on the library transforms: the grid stages of each stream's shapes in sequence on it, so
+  // that small transforms overlap other streams' passes (the same 40 systems: 392 against 467 us a step
+  // stage by stage; 8 systems of 8 shapes: 95 against 104).  One multiply and one interleave per stream, not
+  // per shape, keep the step's graph short: 60 against 68 ms for the first 64 steps, which capture it, and
+  // 417 us a step.  Own passes take all shapes at once.
   if (c->buckets.size() > 1) {
     c->fft_pipeline = 1;
     for (const Bucket& b : c->buckets)

@@ -16,6 +16,7 @@
 //  * stencil weights are recomputed in the gather rather than cached (no ns*S W/inds arrays).
 // Each launch covers every system of the engine: CTAs find their system in a lookup table.
 #include "tild_internal.cuh"
+#include <algorithm>
 #include <climits>
 
 namespace {
@@ -1475,6 +1476,25 @@ int exec_inverse(tild_ctx* c, const Bucket& b) {
   return tild_check_fft(c, cufftExecC2R(b.c2r, c->gk + b.spec0 * c->D, c->gfield + b.grid0 * c->D), "C2R");
 }
 
+// Block ranges (spectrum or grid blocks) of the shapes that `take` accepts, neighbours joined.
+struct Range {
+  int off, n;
+};
+template <class F>
+std::vector<Range> block_ranges(const tild_ctx* c, int Bucket::*first, int Bucket::*count, F&& take) {
+  std::vector<Range> r;
+  for (size_t k = 0; k < c->buckets.size(); k++)
+    if (take(k)) r.push_back({c->buckets[k].*first, c->buckets[k].*count});
+  std::sort(r.begin(), r.end(), [](const Range& a, const Range& b) { return a.off < b.off; });
+  size_t n = 0;
+  for (size_t k = 0; k < r.size(); k++) {
+    if (n && r[n - 1].off + r[n - 1].n == r[k].off) r[n - 1].n += r[k].n;
+    else r[n++] = r[k];
+  }
+  r.resize(n);
+  return r;
+}
+
 int join(tild_ctx* c) {
   for (int k = 0; k < c->lanes; k++) {
     if (tild_check(c, cudaEventRecord(c->ev_join[k], c->aux[k]), "join")) return 1;
@@ -1553,27 +1573,33 @@ int tild_run_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys) {
   }
   c->rho_ahead = false;  // the conversion below clears the accumulator
   if (c->fft_pipeline >= 1 && c->lanes > 0) {
-    // each grid shape runs conversion, R2C, k-space multiply and C2R in order on its stream, so
-    // one shape's transforms overlap another's element-wise passes (one profiling stage)
+    // each stream runs conversion, R2C, k-space multiply, C2R and interleave of its grid shapes in order,
+    // so one stream's transforms overlap another's element-wise passes (one profiling stage)
     tild_mark(c, STAGE_R2C);
     if (fork(c)) return TILD_ERR_CUDA;
-    for (size_t bi = 0; bi < c->buckets.size(); bi++) {
-      const Bucket& b = c->buckets[bi];
-      cudaStream_t bs = b.lane >= 0 ? c->aux[b.lane] : c->stream;
-      if (b.own) {
-        if (tild_fft_run(c, &b, integrate, on[bi], bs)) return TILD_ERR_CUDA;
-        continue;
+    for (int lane = 0; lane < c->lanes; lane++) {
+      cudaStream_t bs = c->aux[lane];
+      auto moves = [&](size_t bi) { return c->buckets[bi].lane == lane && !c->buckets[bi].own && on[bi]; };
+      for (size_t bi = 0; bi < c->buckets.size(); bi++) {
+        const Bucket& b = c->buckets[bi];
+        if (b.lane != lane) continue;
+        if (b.own) {
+          if (tild_fft_run(c, &b, integrate, on[bi], bs)) return TILD_ERR_CUDA;
+          continue;
+        }
+        launch_fix(c, b, bs);
+        if (on[bi] && exec_forward(c, b)) return TILD_ERR_CUDA;
       }
-      launch_fix(c, b, bs);
-      if (!on[bi]) continue;
-      if (exec_forward(c, b)) return TILD_ERR_CUDA;
-      if (c->D == 3) launch_kmul<3>(c, integrate, bs, b.cta_spec0, b.n_cta_spec);
-      else launch_kmul<2>(c, integrate, bs, b.cta_spec0, b.n_cta_spec);
-      c->launches++;
-      if (exec_inverse(c, b))
-        return TILD_ERR_CUDA;
-      if (c->fields.empty()) {  // fieldphase edits the planar fields first when present
-        launch_interleave(c, bs, b.cta_grid0, b.n_cta_grid);
+      for (const Range& r : block_ranges(c, &Bucket::cta_spec0, &Bucket::n_cta_spec, moves)) {
+        if (c->D == 3) launch_kmul<3>(c, integrate, bs, r.off, r.n);
+        else launch_kmul<2>(c, integrate, bs, r.off, r.n);
+        c->launches++;
+      }
+      for (size_t bi = 0; bi < c->buckets.size(); bi++)
+        if (moves(bi) && exec_inverse(c, c->buckets[bi])) return TILD_ERR_CUDA;
+      if (!c->fields.empty()) continue;  // fieldphase edits the planar fields first when present
+      for (const Range& r : block_ranges(c, &Bucket::cta_grid0, &Bucket::n_cta_grid, moves)) {
+        launch_interleave(c, bs, r.off, r.n);
         c->launches++;
       }
     }
@@ -1586,16 +1612,6 @@ int tild_run_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys) {
   bool any_lib = false;
   for (const Bucket& b : c->buckets) any_lib = any_lib || !b.own;
   if (!any_lib) return tild_finish_forces(c, integrate, f_bead, f_sys, true, false);
-  // runs of neighbouring shapes that take the library, in one launch each
-  struct Range { int s0, ns; };
-  std::vector<Range> runs;
-  bool open = false;
-  for (const Bucket& b : c->buckets) {
-    if (b.own) { open = false; continue; }
-    if (!open) runs.push_back({b.cta_spec0, 0});
-    open = true;
-    runs.back().ns += b.n_cta_spec;
-  }
   tild_mark(c, STAGE_ZERO);
   for (const Bucket& b : c->buckets)
     if (!b.own) launch_fix(c, b, c->stream);
@@ -1608,9 +1624,10 @@ int tild_run_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys) {
   }
   if (join(c)) return TILD_ERR_CUDA;
   tild_mark(c, STAGE_KMUL);
-  for (const Range& r : runs) {
-    if (c->D == 3) launch_kmul<3>(c, integrate, c->stream, r.s0, r.ns);
-    else launch_kmul<2>(c, integrate, c->stream, r.s0, r.ns);
+  auto library = [&](size_t bi) { return !c->buckets[bi].own; };
+  for (const Range& r : block_ranges(c, &Bucket::cta_spec0, &Bucket::n_cta_spec, library)) {
+    if (c->D == 3) launch_kmul<3>(c, integrate, c->stream, r.off, r.n);
+    else launch_kmul<2>(c, integrate, c->stream, r.off, r.n);
     c->launches++;
   }
   if (tild_check(c, cudaGetLastError(), "kmul")) return TILD_ERR_CUDA;
@@ -1637,15 +1654,10 @@ int tild_finish_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys, bo
   }
   if (!interleaved) {
     tild_mark(c, STAGE_INTERLEAVE);
-    for (size_t k = 0; k < c->buckets.size();) {  // neighbouring shapes that take the library in one launch
-      const int off = c->buckets[k].cta_grid0;
-      int n = 0;
-      for (; k < c->buckets.size() && !c->buckets[k].own; k++) n += c->buckets[k].n_cta_grid;
-      if (n) {
-        launch_interleave(c, c->stream, off, n);
-        c->launches++;
-      }
-      while (k < c->buckets.size() && c->buckets[k].own) k++;
+    auto library = [&](size_t bi) { return !c->buckets[bi].own; };
+    for (const Range& r : block_ranges(c, &Bucket::cta_grid0, &Bucket::n_cta_grid, library)) {
+      launch_interleave(c, c->stream, r.off, r.n);
+      c->launches++;
     }
   }
   if (!c->fields.empty()) tild_mark(c, STAGE_FIELD);

@@ -294,8 +294,8 @@ typedef struct tild_tune {
   int32_t field_layout;   /* node order of the force field the gather reads: x-fastest (LINEAR) or 4x4x4
                              bricks of consecutive nodes (BRICK, 3D; the box gather needs LINEAR) */
   int32_t fft_pipeline;   /* several grid shapes: 0 runs each stage for all shapes before the next;
-                             1 runs each shape's fixed-point conversion, R2C, k-space multiply, C2R
-                             and interleave in sequence on its own stream; 2 runs each shape's whole
+                             1 runs the fixed-point conversion, R2C, k-space multiply, C2R and interleave
+                             of the shapes of each stream in sequence on it; 2 runs each shape's whole
                              step (spread to gather) on its stream (without fieldphase styles) */
   int32_t spread_ahead;   /* 1: an integrating step's gather (DIRECT) also spreads the updated positions
                              for the next step, which then runs no spread kernel; 0: a spread kernel
