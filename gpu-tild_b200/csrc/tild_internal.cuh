@@ -289,11 +289,10 @@ struct tild_ctx {
   };
   std::vector<TablePlan> tab_plans;
   long long tab_M = 0;
-  bool tab_batch = false;                // a style's force tables and virial kernels are transformed together
+  int tab_nf = 1, tab_nv = 1;            // force tables and virial kernels of a style transformed together
   double* tab_u0 = nullptr;              // u_s(0) of the system's styles
   double* tab_ufull = nullptr;
   cufftDoubleComplex* tab_z = nullptr;
-  cufftDoubleComplex* tab_z2 = nullptr;
   double* tab_freal = nullptr;
   double* tab_vr = nullptr;
 

@@ -9,6 +9,7 @@
 // evaluation stored as FP32; TILD_TABLES_REF_FP32 evaluates the multipliers with the
 // reference's FP32 expressions instead.  Tables cover only the R2C half spectrum.
 #include "tild_internal.cuh"
+#include <algorithm>
 #include <cmath>
 
 namespace {
@@ -253,14 +254,13 @@ int tild_build_tables(tild_ctx* c, int si) {
     if (rc) return rc;
   }
   double* ufull = c->tab_ufull;
-  cufftDoubleComplex* zbuf = c->tab_z;
-  cufftDoubleComplex* zbuf2 = c->tab_z2;
+  cufftDoubleComplex* zbuf = c->tab_z;  // of the force tables, then of the virial kernels
   double* freal = c->tab_freal;
   double* vr = c->tab_vr;
   SysDev& hd = c->h_sys[si];
   // the D force tables and nP virial kernels of a style go through the transforms together (one by one
   // their launches were most of the 685 us of loading a slot)
-  const int nf = c->tab_batch ? D : 1, nv = c->tab_batch ? h.nP : 1;
+  const int nf = c->tab_nf, nv = c->tab_nv;
   double u0[TILD_MAX_STYLES];
   for (int s = 0; s < nfft && rc == TILD_OK; s++) {
     const tild_pair_style& ps = h.cfg.styles[h.fft_cfg[s]];
@@ -286,8 +286,8 @@ int tild_build_tables(tild_ctx* c, int si) {
     for (int j = 0; j < h.nP && rc == TILD_OK; j += nv) {
       k_virial_real<<<dim3(nblk(g.M, 256), nv), 256, 0, st>>>(vr, freal, g, D, Mpad, j);
       c->launches++;
-      if (tild_check_fft(c, cufftExecD2Z(pd2z, vr, zbuf2), "exec d2z")) { rc = TILD_ERR_CUDA; break; }
-      k_store_virk<<<dim3(nblk(g.Mh, 256), nv), 256, 0, st>>>(c->virk + h.virk0 + ((long long)s * h.nP + j) * g.Mh, zbuf2, g.Mh,
+      if (tild_check_fft(c, cufftExecD2Z(pd2z, vr, zbuf), "exec d2z")) { rc = TILD_ERR_CUDA; break; }
+      k_store_virk<<<dim3(nblk(g.Mh, 256), nv), 256, 0, st>>>(c->virk + h.virk0 + ((long long)s * h.nP + j) * g.Mh, zbuf, g.Mh,
                                                               invM * invM);
       c->launches++;
     }
@@ -324,13 +324,16 @@ int tild_table_scratch(tild_ctx* c) {
     D = h.D;
   }
   const long long Mpad = (M + 1) / 2 * 2;
-  // whole styles at a time up to 2^21 points (0.4 GB of scratch at 128^3), above that one table
-  c->tab_batch = M <= (1ll << 21);
-  const int nf = c->tab_batch ? D : 1, nv = c->tab_batch ? (D == 3 ? 6 : 3) : 1;
+  // Whole styles at a time up to 2^18 points, where launches count (loading a slot 0.74 -> 0.36 ms at 24^3 to
+  // 48^3, 0.90 -> 0.46 at 64^3); half of the virial kernels together up to 2^21, where the scratch does
+  // (a 128^3 system with three styles takes 644 MB in all, 847 with all six and 528 one by one, and loads in
+  // 1.69, 1.65 and 2.00 ms); above that one table.
+  c->tab_nf = M <= (1ll << 21) ? D : 1;
+  c->tab_nv = D == 3 && M <= (1ll << 18) ? 6 : M <= (1ll << 21) ? 3 : 1;
+  const int nf = c->tab_nf, nv = c->tab_nv;
   if (tild_check(c, cudaMalloc(&c->tab_ufull, sizeof(double) * Mh), "alloc table scratch") ||
       tild_check(c, cudaMalloc(&c->tab_u0, sizeof(double) * TILD_MAX_STYLES), "alloc table scratch") ||
-      tild_check(c, cudaMalloc(&c->tab_z, sizeof(cufftDoubleComplex) * Mh * nf), "alloc table scratch") ||
-      tild_check(c, cudaMalloc(&c->tab_z2, sizeof(cufftDoubleComplex) * Mh * nv), "alloc table scratch") ||
+      tild_check(c, cudaMalloc(&c->tab_z, sizeof(cufftDoubleComplex) * Mh * std::max(nf, nv)), "alloc table scratch") ||
       tild_check(c, cudaMalloc(&c->tab_freal, sizeof(double) * Mpad * D), "alloc table scratch") ||
       tild_check(c, cudaMalloc(&c->tab_vr, sizeof(double) * Mpad * nv), "alloc table scratch"))
     return TILD_ERR_OOM;
@@ -353,7 +356,7 @@ int tild_table_plans(tild_ctx* c, const Geom& g, int D, cufftHandle* z2d, cufftH
   for (int q = 0; q < 3; q++) tp.nx[q] = g.nx[q];
   tp.z2d = tp.d2z = 0;
   // complex lines Mh apart, real ones on 16-byte boundaries
-  const int nf = c->tab_batch ? D : 1, nv = c->tab_batch ? (D == 3 ? 6 : 3) : 1;
+  const int nf = c->tab_nf, nv = c->tab_nv;
   const int Mpad = (int)((g.M + 1) / 2 * 2), Mh = (int)g.Mh;
   int real[3], half[3];
   for (int q = 0; q < D; q++) real[q] = half[q] = n[q];
@@ -382,10 +385,10 @@ void tild_tables_free(tild_ctx* c) {
     cufftDestroy(tp.d2z);
   }
   c->tab_plans.clear();
-  void* ptrs[] = {c->tab_ufull, c->tab_u0, c->tab_z, c->tab_z2, c->tab_freal, c->tab_vr};
+  void* ptrs[] = {c->tab_ufull, c->tab_u0, c->tab_z, c->tab_freal, c->tab_vr};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   c->tab_ufull = c->tab_u0 = nullptr;
-  c->tab_z = c->tab_z2 = nullptr;
+  c->tab_z = nullptr;
   c->tab_freal = c->tab_vr = nullptr;
 }
