@@ -352,6 +352,14 @@ struct Lines {
       : nx(g.nx[0]), ny(D == 3 ? g.nx[1] : 1), nz(D == 3 ? g.nx[2] : g.nx[1]), M(g.M) {}
 };
 
+// active_at with its three reads under way together: their latency is on the path of every pass (40^3:
+// 28.7 us a step, one after another 29.6).  past: `ahead`, or kFirstStep in place of 0.
+constexpr int kFirstStep = -(1 << 30);
+__device__ __forceinline__ bool moves(const SysDev* sd, int past) {
+  const long long stop = sd->stop_at, step = sd->step;
+  return sd->active && (stop < 0 || step + past < stop);
+}
+
 // rows of an x pass's CTA: about `points` points of each field
 __host__ __device__ inline int rows_per_cta(int nx, int points) {
   return points < nx ? 1 : points / nx > 32 ? 32 : points / nx;
@@ -364,7 +372,7 @@ __host__ __device__ inline int rows_per_cta(int nx, int points) {
 __global__ void __launch_bounds__(kThreads, kMinCtas) k_fft_x_fwd(unsigned long long* __restrict__ fx, float* __restrict__ rho,
                                                    float2* __restrict__ zk, const float2* __restrict__ twid,
                                                    const int2* __restrict__ blocks, const SysDev* __restrict__ sysd,
-                                                   int D, int points, int write_rho, int ahead, int blk_off) {
+                                                   int D, int points, int write_rho, int past, int blk_off) {
   extern __shared__ __align__(16) float2 ex[];
   const int2 bk = blocks[blockIdx.x + blk_off];
   const SysDev& sd = sysd[bk.x];
@@ -380,7 +388,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) k_fft_x_fwd(unsigned long 
   ra += (long long)row0 * g.nx;
   grid_launch_next();
   grid_wait();
-  const bool act = active_at(*after_wait(&sd), ahead);
+  const bool act = moves(after_wait(&sd), past);
   a = after_wait(a);
   unsigned long long* b = a + g.M;
   // the rows are one run of the grid: coalesced loads, kXBatch of each channel in flight per thread
@@ -454,7 +462,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) k_fft_x_fwd(unsigned long 
 template <bool DIRECT>
 __global__ void __launch_bounds__(kThreads, kMinCtas) k_fft_y_fwd(float2* __restrict__ zk, const float2* __restrict__ twid,
                                                    const int2* __restrict__ blocks, const SysDev* __restrict__ sysd,
-                                                   int ahead, int blk_off) {
+                                                   int past, int blk_off) {
   extern __shared__ __align__(16) float2 ex[];
   constexpr int LT = kColsFwd;
   const int2 bk = blocks[blockIdx.x + blk_off];
@@ -470,7 +478,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) k_fft_y_fwd(float2* __rest
   char* z = reinterpret_cast<char*>(zk + sd.zk0 + (long long)p * g.M + (long long)cz * g.nx * g.ny + (c - cz * g.nx));
   grid_launch_next();
   grid_wait();
-  if (!active_at(*after_wait(&sd), ahead)) return;
+  if (!moves(after_wait(&sd), past)) return;
   z = after_wait(z);
   with_radix(R1, [&](auto rc) {
     constexpr int R = decltype(rc)::value;
@@ -620,7 +628,7 @@ __global__ void __launch_bounds__(kThreadsZ, kMinCtasZ) k_fft_z_kmul(const float
   grid_launch_next();  // only now: what starts early from here on (the gather) finds the last step's kernels done
   const SysDev* now = after_wait(&sd);
   const long long est = now->step + ahead + (integrate ? 1 : 0);
-  if (!active_at(*now, ahead)) return;
+  if (!moves(now, ahead ? ahead : kFirstStep)) return;
   zk = after_wait(zk);
   if (tile && threadIdx.x < nu) s_scale[threadIdx.x] = sd.zramp[threadIdx.x] < 0 ? 1.f : ramp_ratio(sd, sd.zramp[threadIdx.x], est);
   for (int p0 = 0; p0 < np; p0 += 2) {
@@ -754,7 +762,7 @@ struct Field {
 template <int LT, bool DIRECT>
 __global__ void __launch_bounds__(LT == 8 ? 192 : 128, LT == 8 ? 5 : 8)
     k_fft_y_inv(float2* __restrict__ gk, const float* __restrict__ kd_all, const float2* __restrict__ twid,
-                const int2* __restrict__ blocks, const SysDev* __restrict__ sysd, int ahead, int blk_off) {
+                const int2* __restrict__ blocks, const SysDev* __restrict__ sysd, int past, int blk_off) {
   extern __shared__ __align__(16) float2 ex[];
   constexpr int THREADS = LT == 8 ? 192 : 128, NF = LT == 8 ? 3 : 1;  // NF fields at once
   const int2 bk = blocks[blockIdx.x + blk_off];
@@ -775,7 +783,7 @@ __global__ void __launch_bounds__(LT == 8 ? 192 : 128, LT == 8 ? 5 : 8)
   const FastDiv dr(R2), df(nq);
   grid_launch_next();
   grid_wait();
-  if (!active_at(*after_wait(&sd), ahead)) return;
+  if (!moves(after_wait(&sd), past)) return;
   z = after_wait(z);
   // P's y derivative first: P itself is overwritten by its x derivative
   for (int f0 = 0; f0 < 3; f0 += NF) {
@@ -825,7 +833,7 @@ __global__ void __launch_bounds__(LT == 8 ? 192 : 128, LT == 8 ? 5 : 8)
 template <bool DIRECT>
 __global__ void __launch_bounds__(kThreadsX, kMinCtasX) k_fft_x_inv(const float2* __restrict__ gk, float4* __restrict__ g4_all,
                                                    const float2* __restrict__ twid, const int2* __restrict__ blocks,
-                                                   const SysDev* __restrict__ sysd, int D, int points, int layout, int ahead, int blk_off) {
+                                                   const SysDev* __restrict__ sysd, int D, int points, int layout, int past, int blk_off) {
   extern __shared__ __align__(16) float2 ex[];
   __shared__ int s_row[32];  // node offset of each row
   const int2 bk = blocks[blockIdx.x + blk_off];
@@ -845,7 +853,7 @@ __global__ void __launch_bounds__(kThreadsX, kMinCtasX) k_fft_x_inv(const float2
   }
   grid_launch_next();
   grid_wait();
-  if (!active_at(*after_wait(&sd), ahead)) return;
+  if (!moves(after_wait(&sd), past)) return;
   src = after_wait(src);
   with_radix(R1, [&](auto rc) {
     constexpr int R = decltype(rc)::value;
@@ -909,7 +917,7 @@ template <bool DIRECT>
 __global__ void __launch_bounds__(kThreadsPlane, 1024 / kThreadsPlane)
     k_fft_plane_fwd(unsigned long long* __restrict__ fx, float* __restrict__ rho, float2* __restrict__ zk,
                     const float2* __restrict__ twid, const int2* __restrict__ blocks, const SysDev* __restrict__ sysd,
-                    int write_rho, int ahead, int blk_off) {
+                    int write_rho, int past, int blk_off) {
   extern __shared__ __align__(16) float2 ex[];
   const int2 bk = blocks[blockIdx.x + blk_off];
   const SysDev& sd = sysd[bk.x];
@@ -926,7 +934,7 @@ __global__ void __launch_bounds__(kThreadsPlane, 1024 / kThreadsPlane)
   ra += (long long)plane * npt;
   grid_launch_next();
   grid_wait();
-  const bool act = active_at(*after_wait(&sd), ahead);
+  const bool act = moves(after_wait(&sd), past);
   a = after_wait(a);
   unsigned long long* b = a + g.M;
   for (int i0 = threadIdx.x; i0 < npt; i0 += kXBatch * kThreadsPlane) {
@@ -1015,7 +1023,7 @@ template <int THREADS, bool DIRECT>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
     k_fft_plane_inv(const float2* __restrict__ gk, float4* __restrict__ g4_all, const float* __restrict__ kd_all,
                     const float2* __restrict__ twid, const int2* __restrict__ blocks, const SysDev* __restrict__ sysd,
-                    int layout, int ahead, int blk_off) {
+                    int layout, int past, int blk_off) {
   extern __shared__ __align__(16) float2 ex[];
   const int2 bk = blocks[blockIdx.x + blk_off];
   const SysDev& sd = sysd[bk.x];
@@ -1030,7 +1038,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
   const FastDiv dj(R2), dk(R1), dx(nx);
   grid_launch_next();
   grid_wait();
-  if (!active_at(*after_wait(&sd), ahead)) return;
+  if (!moves(after_wait(&sd), past)) return;
   src = after_wait(src);
   with_radix(Y1, [&](auto rc) {
     constexpr int R = decltype(rc)::value;
@@ -1332,20 +1340,20 @@ int tild_fft_run(tild_ctx* c, const Bucket* b, bool integrate, bool active, cuda
   float2* zk = reinterpret_cast<float2*>(c->rhok);
   float2* gk = reinterpret_cast<float2*>(c->gk);
   const auto* pa = c->fft_pass;
-  const int wr = !integrate || c->last_of_call || !c->fields.empty(), ahead = c->ahead;
+  const int wr = !integrate || c->last_of_call || !c->fields.empty(), ahead = c->ahead, past = ahead ? ahead : kFirstStep;
   const bool* dir = b ? b->fft_direct : c->fft_direct;
   if (!b) tild_mark(c, STAGE_ZERO);
   if (c->fft_plane)
     tild_launch_early(dir[0] || dir[1] ? k_fft_plane_fwd<true> : k_fft_plane_fwd<false>, n[0], kThreadsPlane, pa[0].smem, kCarveout, st, c->rho_fx, c->rho, zk, c->fft_twid, pa[0].blocks,
-                      c->d_sys, wr, ahead, off[0]);
+                      c->d_sys, wr, past, off[0]);
   else
-    tild_launch_early(k_fft_x_fwd, n[0], kThreads, pa[0].smem, kCarveout, st, c->rho_fx, c->rho, zk, c->fft_twid, pa[0].blocks, c->d_sys, c->D, c->fft_points, wr, ahead, off[0]);
+    tild_launch_early(k_fft_x_fwd, n[0], kThreads, pa[0].smem, kCarveout, st, c->rho_fx, c->rho, zk, c->fft_twid, pa[0].blocks, c->d_sys, c->D, c->fft_points, wr, past, off[0]);
   c->launches++;
   if (!active) return tild_check(c, cudaGetLastError(), "grid passes");  // no system of the shape moves: densities only
   const bool columns = c->D == 3 && !c->fft_plane;
   if (columns) {
     if (!b) tild_mark(c, STAGE_R2C);
-    tild_launch_early(dir[1] ? k_fft_y_fwd<true> : k_fft_y_fwd<false>, n[1], kThreads, pa[1].smem, kCarveout, st, zk, c->fft_twid, pa[1].blocks, c->d_sys, ahead, off[1]);
+    tild_launch_early(dir[1] ? k_fft_y_fwd<true> : k_fft_y_fwd<false>, n[1], kThreads, pa[1].smem, kCarveout, st, zk, c->fft_twid, pa[1].blocks, c->d_sys, past, off[1]);
     c->launches++;
   }
   if (!b) tild_mark(c, STAGE_KMUL);
@@ -1354,9 +1362,9 @@ int tild_fft_run(tild_ctx* c, const Bucket* b, bool integrate, bool active, cuda
   if (columns) {
     if (!b) tild_mark(c, STAGE_C2R);
     if (c->fft_wide)
-      tild_launch_early(dir[1] ? k_fft_y_inv<16, true> : k_fft_y_inv<16, false>, n[3], 128, pa[3].smem, kCarveout, st, gk, c->kd, c->fft_twid, pa[3].blocks, c->d_sys, ahead, off[3]);
+      tild_launch_early(dir[1] ? k_fft_y_inv<16, true> : k_fft_y_inv<16, false>, n[3], 128, pa[3].smem, kCarveout, st, gk, c->kd, c->fft_twid, pa[3].blocks, c->d_sys, past, off[3]);
     else
-      tild_launch_early(dir[1] ? k_fft_y_inv<8, true> : k_fft_y_inv<8, false>, n[3], 192, pa[3].smem, kCarveout, st, gk, c->kd, c->fft_twid, pa[3].blocks, c->d_sys, ahead, off[3]);
+      tild_launch_early(dir[1] ? k_fft_y_inv<8, true> : k_fft_y_inv<8, false>, n[3], 192, pa[3].smem, kCarveout, st, gk, c->kd, c->fft_twid, pa[3].blocks, c->d_sys, past, off[3]);
     c->launches++;
   }
   if (!b) tild_mark(c, STAGE_INTERLEAVE);
@@ -1364,9 +1372,9 @@ int tild_fft_run(tild_ctx* c, const Bucket* b, bool integrate, bool active, cuda
     tild_launch_early(dir[0] || dir[1] ? (n[4] <= 296 ? k_fft_plane_inv<512, true> : k_fft_plane_inv<256, true>)
                                        : (n[4] <= 296 ? k_fft_plane_inv<512, false> : k_fft_plane_inv<256, false>),
                       n[4], n[4] <= 296 ? 512 : 256, pa[4].smem, kCarveout, st, gk, c->g4, c->kd, c->fft_twid, pa[4].blocks,
-                      c->d_sys, c->field_layout, ahead, off[4]);
+                      c->d_sys, c->field_layout, past, off[4]);
   else
-    tild_launch_early(dir[0] ? k_fft_x_inv<true> : k_fft_x_inv<false>, n[4], kThreadsX, pa[4].smem, kCarveout, st, gk, c->g4, c->fft_twid, pa[4].blocks, c->d_sys, c->D, c->fft_points, c->field_layout, ahead, off[4]);
+    tild_launch_early(dir[0] ? k_fft_x_inv<true> : k_fft_x_inv<false>, n[4], kThreadsX, pa[4].smem, kCarveout, st, gk, c->g4, c->fft_twid, pa[4].blocks, c->d_sys, c->D, c->fft_points, c->field_layout, past, off[4]);
   c->launches += 2;
   return tild_check(c, cudaGetLastError(), "grid passes");
 }

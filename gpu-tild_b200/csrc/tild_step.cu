@@ -144,7 +144,7 @@ __device__ __forceinline__ void cta_spread_box(bool ok, const float (&xs)[3], in
     float Wd[P + 1];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-      s_g0[d] = (ok && d < D) ? axis_base<P>(xs[d], g.dx[d], g.rdx[d], Wd) : 0;
+      s_g0[d] = (ok && d < D) ? axis_base<P, false>(xs[d], g.dx[d], g.rdx[d], Wd) : 0;
       s_min[d] = INT_MAX;
       s_max[d] = INT_MIN;
     }
@@ -155,7 +155,7 @@ __device__ __forceinline__ void cta_spread_box(bool ok, const float (&xs)[3], in
   int rel[3] = {0, 0, 0};
   if (ok) {
 #pragma unroll
-    for (int d = 0; d < D; d++) rel[d] = fold_rel(axis_index<P>(xs[d], g.dx[d], g.rdx[d], gd[d]) - s_g0[d], g.nx[d]);
+    for (int d = 0; d < D; d++) rel[d] = fold_rel(axis_index<P, false>(xs[d], g.dx[d], g.rdx[d], gd[d]) - s_g0[d], g.nx[d]);
   }
   int mn[3], ext[3];
   long long vol;
@@ -255,7 +255,7 @@ __device__ __forceinline__ void bead_spread_direct(const float (&xs)[3], int t, 
   int idx[3][P + 1];
 #pragma unroll
   for (int d = 0; d < D; d++) {
-    const int b = axis_base<P>(xs[d], g.dx[d], g.rdx[d], W[d]);
+    const int b = axis_base<P, false>(xs[d], g.dx[d], g.rdx[d], W[d]);
 #pragma unroll
     for (int a = 0; a <= P; a++) idx[d][a] = pmod(b + a, g.nx[d]);
   }
