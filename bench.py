@@ -322,6 +322,14 @@ def stage_bytes(s, passes: bool = True) -> dict:
     }
 
 
+def stage_names(s) -> dict:
+    """What the grid stages of a system on the library's own passes run: lines along one axis each, or the
+    x and y passes of a plane of up to 2,304 points in one kernel (the stages between are then empty)."""
+    planes = s.dim == 3 and s.nx[0] * s.nx[1] <= 2304
+    return {"fix2float": "xy_forward" if planes else "x_forward", "r2c": "y_forward", "kmul": "z_multiply",
+            "c2r": "y_inverse", "interleave": "xy_inverse" if planes else "x_inverse"}
+
+
 def step_bytes(s) -> int:
     """Compulsory bytes of one whole step of a fused design: ns * b_p + M * 48 * channels, with
     b_p = 104 B per bead for GJF (64 for EM, +4 with charges)."""
@@ -430,7 +438,7 @@ def run_ours(args):
 
     # per-stage times over the same number of steps -> roofline of the dominant kernel
     prof = ctx.profile_steps(args.steps)
-    sb = stage_bytes(s)
+    sb, names = stage_bytes(s), stage_names(s)
     dom = max(prof, key=lambda k: prof[k])
     dom_ms = prof[dom] / args.steps
     peak, peak_kind = hbm_peak()
@@ -488,8 +496,8 @@ def run_ours(args):
         "clocks": clocks,
         "e2e": e2e,
         "gpu_launches": int(launches),
-        "stages_ms_per_step": {k: v / args.steps for k, v in prof.items()},
-        "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "GB/s",
+        "stages_ms_per_step": {names.get(k, k): v / args.steps for k, v in prof.items()},
+        "roofline": {"bound": "hbm", "kernel": names.get(dom, dom), "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_source": f"{peak_kind} ({'MEASURED_PEAKS.json' if peak_kind == 'measured' else 'fallback'})",
                      "algorithmic_bytes_per_launch": sb[dom],
                      "traffic": NCU_DRAM_BYTES_PER_LAUNCH.get(wname, {}).get(dom)},

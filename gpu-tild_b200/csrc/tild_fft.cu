@@ -1201,11 +1201,11 @@ int tild_fft_setup(tild_ctx* c) {
   for (const Bucket& b : c->buckets)
     for (int s : b.systems)
       if (b.own) points += (c->sys[s].T + c->sys[s].C + 1) / 2 * c->sys[s].g.M;
-  c->fft_points = (int)std::min(1024ll, std::max(256ll, points / 592));
+  c->fft_points = (int)std::min(1024ll, std::max(256ll, points / (4 * kSms)));
   c->fft_plane = D == 3;
   for (const Bucket& b : c->buckets)
     if (b.own) c->fft_plane = c->fft_plane && b.nx[0] * b.nx[1] <= kPlanePoints;
-  c->fft_wide = points >= 16 * 32 * 592;  // the y inverse pass still has some CTAs of 16 columns for every SM
+  c->fft_wide = points >= 16 * 32 * 4 * kSms;  // the y inverse pass still has some CTAs of 16 columns for every SM
   std::vector<int2> tab[5];
   long long ztotal = 0;
   for (Bucket& b : c->buckets) {
@@ -1342,6 +1342,7 @@ int tild_fft_run(tild_ctx* c, const Bucket* b, bool integrate, bool active, cuda
   const auto* pa = c->fft_pass;
   const int wr = !integrate || c->last_of_call || !c->fields.empty(), ahead = c->ahead, past = ahead ? ahead : kFirstStep;
   const bool* dir = b ? b->fft_direct : c->fft_direct;
+  const bool few = n[4] <= 2 * kSms;  // planes' fields
   if (!b) tild_mark(c, STAGE_ZERO);
   if (c->fft_plane)
     tild_launch_early(dir[0] || dir[1] ? k_fft_plane_fwd<true> : k_fft_plane_fwd<false>, n[0], kThreadsPlane, pa[0].smem, kCarveout, st, c->rho_fx, c->rho, zk, c->fft_twid, pa[0].blocks,
@@ -1369,9 +1370,9 @@ int tild_fft_run(tild_ctx* c, const Bucket* b, bool integrate, bool active, cuda
   }
   if (!b) tild_mark(c, STAGE_INTERLEAVE);
   if (c->fft_plane)
-    tild_launch_early(dir[0] || dir[1] ? (n[4] <= 296 ? k_fft_plane_inv<512, true> : k_fft_plane_inv<256, true>)
-                                       : (n[4] <= 296 ? k_fft_plane_inv<512, false> : k_fft_plane_inv<256, false>),
-                      n[4], n[4] <= 296 ? 512 : 256, pa[4].smem, kCarveout, st, gk, c->g4, c->kd, c->fft_twid, pa[4].blocks,
+    tild_launch_early(dir[0] || dir[1] ? (few ? k_fft_plane_inv<512, true> : k_fft_plane_inv<256, true>)
+                                       : (few ? k_fft_plane_inv<512, false> : k_fft_plane_inv<256, false>),
+                      n[4], few ? 512 : 256, pa[4].smem, kCarveout, st, gk, c->g4, c->kd, c->fft_twid, pa[4].blocks,
                       c->d_sys, c->field_layout, past, off[4]);
   else
     tild_launch_early(dir[0] ? k_fft_x_inv<true> : k_fft_x_inv<false>, n[4], kThreadsX, pa[4].smem, kCarveout, st, gk, c->g4, c->fft_twid, pa[4].blocks, c->d_sys, c->D, c->fft_points, c->field_layout, past, off[4]);

@@ -392,6 +392,8 @@ inline void tild_launch_early(void (*kernel)(P...), int grid, int threads, size_
   cfg.numAttrs = carveout < 0 ? 1 : 2;
   cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
+constexpr int kSms = 148;  // of a B200: launches are judged by their CTAs per SM
+
 // One shared-memory split for the passes of a step: an SM that has to change its split between two
 // kernels drains first, so the next one could not start early there (40^3, 40,000 beads: 36.3 us a step
 // with one split for the grid passes, 46.4 with the driver's choice for each, 39 without early starts).

@@ -1235,7 +1235,7 @@ inline BeadRange all_beads(tild_ctx* c) { return {c->stream, 0, c->n_cta_bead}; 
 // a CTA clear and flush more words a bead (2.6M blend 126 and 337 us), except in systems that do not fill
 // the SMs (10,000 beads: 10.0 and 7.5 us; 60,000 of order 4: 26 and 20).
 int spread_share(const tild_ctx* c) {
-  if (c->n_cta_bead < 296) return 4;
+  if (c->n_cta_bead < 2 * kSms) return 4;
   int share = 1;
   for (const SysHost& h : c->sys) {
     const double density = (double)h.ns / (double)h.g.M;
@@ -1294,7 +1294,7 @@ void launch_gather_k(tild_ctx* c, float* f_out, int f_sys, BeadRange r) {
   }
   if constexpr (I && !X && P <= 1) {
     const bool ahead = tild_spreads_ahead(c, true);
-    if (r.n < 296) {  // 2 CTAs per SM
+    if (r.n < 2 * kSms) {
       auto early = [&](auto* kernel, unsigned long long* rho_fx) {
         tild_launch_early(kernel, r.n, kTile, 0, kCarveout, r.st, c->pos[c->cur], c->pos[c->cur ^ 1], c->noise, c->bead_id,
                           c->bond_nbr, c->bond_info, c->charge, c->g4, c->cta_bead, c->d_sys, f_out, f_sys, c->xorwow,

@@ -24,7 +24,8 @@ by memory, not by a fixed number of slots per shape.  The loop
 
 A job's result does not depend on what else runs or which pool holds it: the spread is fixed
 point (order-independent), the noise is keyed by (bead id, step, seed), and every other kernel is
-per bead or per grid point of one system.  Only cuFFT's batched transforms could round
+per bead, per grid line or per grid point of one system.  Only cuFFT's batched transforms (of the
+energies and S(k), and of the step on grid shapes that the own passes do not take) could round
 differently with the batch size; the serving test bounds that.
 """
 from __future__ import annotations
