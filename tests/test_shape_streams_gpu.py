@@ -42,3 +42,19 @@ def test_streams_of_several_shapes(streams, fieldphase):
             out.append([B.get_state(i)[0] for i in range(len(systems))] + [B.density(i) for i in range(len(systems))] + [f])
     for k, (a, b) in enumerate(zip(*out)):
         assert np.array_equal(a, b), k
+
+
+def test_large_batches_go_shape_by_shape():
+    """Above 150 MB of spectra and force spectra each shape of a stream launches its own multiply and interleave."""
+    shapes = [(96, 96, 96), (100, 96, 96), (96, 100, 96), (96, 96, 100), (100, 100, 96)]
+    systems = [small_diblock(3, 1, nx=n, box=tuple(0.5 * v for v in n), n_chains=300, seed=k) for k, n in enumerate(shapes)]
+    out = []
+    for pipeline in (0, 1):
+        with tild.Batch(systems) as B:
+            t = B.get_tune()
+            t.fft_pipeline, t.fft_streams = pipeline, 2
+            B.set_tune(t)
+            B.step(9)
+            out.append([B.get_state(i)[0] for i in range(5)])
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
