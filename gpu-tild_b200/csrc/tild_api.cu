@@ -657,9 +657,7 @@ int engine_create(const tild_config* cfgs, int nsys, int device, tild_ctx* c, co
   if (tild_assign_lanes(c, (int)c->aux.size())) return TILD_ERR_CUDA;
   // several shapes on the library transforms: the grid stages of each stream's shapes in sequence on it, so
   // that small transforms overlap other streams' passes (the same 40 systems: 392 against 467 us a step
-  // stage by stage; 8 systems of 8 shapes: 95 against 104).  One multiply and one interleave per stream, not
-  // per shape, keep the step's graph short: 60 against 68 ms for the first 64 steps, which capture it, and
-  // 417 us a step.  Own passes take all shapes at once.
+  // stage by stage; 8 systems of 8 shapes: 95 against 104).  Own passes take all shapes at once.
   if (c->buckets.size() > 1) {
     c->fft_pipeline = 1;
     for (const Bucket& b : c->buckets)

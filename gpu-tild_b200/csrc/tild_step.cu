@@ -26,7 +26,7 @@ inline unsigned nblk(long long n, int b) { return (unsigned)((n + b - 1) / b); }
 constexpr double kInvFix = 1.0 / 4294967296.0;  // the global accumulator holds 2^32 per unit
 constexpr int kMaxRows = 1024;                  // (y, z) rows of a shared-memory spread box
 constexpr int kSortForcesSlots = 100000;        // slots from which force-only evaluations sort the beads
-constexpr long long kGroupBytes = 150ll << 20;  // spectra and force spectra of a batch whose streams' shapes share launches
+constexpr long long kGroupBytes = 256ll << 20;  // spectra and force spectra of a batch whose streams' shapes share launches
 constexpr int kGatherBoxMax = 3072;             // float4 nodes of the gather's shared box (48 KB)
 
 // n mod N in [0, N); indices within one period of the grid (nearly all) take no division
@@ -1576,42 +1576,41 @@ int tild_run_forces(tild_ctx* c, bool integrate, float* f_bead, int f_sys) {
   if (c->fft_pipeline >= 1 && c->lanes > 0) {
     // each stream runs conversion, R2C, k-space multiply, C2R and interleave of its grid shapes in order,
     // so one stream's transforms overlap another's element-wise passes (one profiling stage).  All shapes
-    // of a stream go together through the multiply and the interleave while most of the batch's fields stay
-    // in L2 between them; in larger batches each shape by itself keeps what it hands on there.  us a step on 8
-    // streams, shape by shape / together: 20 ensemble systems 237 / 217, 40 452 / 424, 60 (105 MB) 616 / 595,
-    // 80 (140 MB) 713 / 708, 100 (175 MB) 887 / 891, 256 on 4 streams 2,199 / 2,236.
+    // of a stream go together through the multiply and the interleave, which shortens the step's graph; in
+    // large batches each shape by itself, which keeps what it hands on in L2.  us a step on 8 streams, shape
+    // by shape / together: 20 ensemble systems 237 / 217, 40 452 / 424, 80 (140 MB) 713 / 708, 100 (175 MB)
+    // 909 / 913 and 93 / 88 ms for the first 64 steps, which capture the graph; 256 (440 MB) 2,290 / 2,306,
+    // on 4 streams 2,190 / 2,231.
     tild_mark(c, STAGE_R2C);
     if (fork(c)) return TILD_ERR_CUDA;
     const bool grouped = (c->D + 1) * c->spec_total * (long long)sizeof(float2) <= kGroupBytes;
-    for (int lane = 0; lane < c->lanes; lane++) {
+    const size_t n = c->buckets.size(), groups = grouped ? c->lanes : n;
+    for (size_t g = 0; g < groups; g++) {  // the shapes of a stream, or one shape
+      const int lane = grouped ? (int)g : c->buckets[g].lane;
       cudaStream_t bs = c->aux[lane];
-      const size_t n = c->buckets.size();
-      for (size_t b0 = 0; b0 < n; b0 = grouped ? n : b0 + 1) {  // shapes b0 to b1 - 1 of the stream
-        const size_t b1 = grouped ? n : b0 + 1;
-        auto mine = [&](size_t bi) { return bi >= b0 && bi < b1 && c->buckets[bi].lane == lane; };
-        auto moves = [&](size_t bi) { return mine(bi) && !c->buckets[bi].own && on[bi]; };
-        for (size_t bi = b0; bi < b1; bi++) {
-          const Bucket& b = c->buckets[bi];
-          if (!mine(bi)) continue;
-          if (b.own) {
-            if (tild_fft_run(c, &b, integrate, on[bi], bs)) return TILD_ERR_CUDA;
-            continue;
-          }
-          launch_fix(c, b, bs);
-          if (on[bi] && exec_forward(c, b)) return TILD_ERR_CUDA;
+      auto mine = [&](size_t bi) { return grouped ? c->buckets[bi].lane == lane : bi == g; };
+      auto moves = [&](size_t bi) { return mine(bi) && !c->buckets[bi].own && on[bi]; };
+      for (size_t bi = 0; bi < n; bi++) {
+        const Bucket& b = c->buckets[bi];
+        if (!mine(bi)) continue;
+        if (b.own) {
+          if (tild_fft_run(c, &b, integrate, on[bi], bs)) return TILD_ERR_CUDA;
+          continue;
         }
-        for (const Range& r : block_ranges(c, &Bucket::cta_spec0, &Bucket::n_cta_spec, moves)) {
-          if (c->D == 3) launch_kmul<3>(c, integrate, bs, r.off, r.n);
-          else launch_kmul<2>(c, integrate, bs, r.off, r.n);
-          c->launches++;
-        }
-        for (size_t bi = b0; bi < b1; bi++)
-          if (moves(bi) && exec_inverse(c, c->buckets[bi])) return TILD_ERR_CUDA;
-        if (!c->fields.empty()) continue;  // fieldphase edits the planar fields first when present
-        for (const Range& r : block_ranges(c, &Bucket::cta_grid0, &Bucket::n_cta_grid, moves)) {
-          launch_interleave(c, bs, r.off, r.n);
-          c->launches++;
-        }
+        launch_fix(c, b, bs);
+        if (on[bi] && exec_forward(c, b)) return TILD_ERR_CUDA;
+      }
+      for (const Range& r : block_ranges(c, &Bucket::cta_spec0, &Bucket::n_cta_spec, moves)) {
+        if (c->D == 3) launch_kmul<3>(c, integrate, bs, r.off, r.n);
+        else launch_kmul<2>(c, integrate, bs, r.off, r.n);
+        c->launches++;
+      }
+      for (size_t bi = 0; bi < n; bi++)
+        if (moves(bi) && exec_inverse(c, c->buckets[bi])) return TILD_ERR_CUDA;
+      if (!c->fields.empty()) continue;  // fieldphase edits the planar fields first when present
+      for (const Range& r : block_ranges(c, &Bucket::cta_grid0, &Bucket::n_cta_grid, moves)) {
+        launch_interleave(c, bs, r.off, r.n);
+        c->launches++;
       }
     }
     if (join(c)) return TILD_ERR_CUDA;

@@ -45,8 +45,8 @@ def test_streams_of_several_shapes(streams, fieldphase):
 
 
 def test_large_batches_go_shape_by_shape():
-    """Above 150 MB of spectra and force spectra each shape of a stream launches its own multiply and interleave."""
-    shapes = [(96, 96, 96), (100, 96, 96), (96, 100, 96), (96, 96, 100), (100, 100, 96)]
+    """Above 256 MB of spectra and force spectra each shape of a stream launches its own multiply and interleave."""
+    shapes = [(120, 120, 120), (125, 120, 120), (120, 125, 120), (120, 120, 125), (125, 125, 120)]
     systems = [small_diblock(3, 1, nx=n, box=tuple(0.5 * v for v in n), n_chains=300, seed=k) for k, n in enumerate(shapes)]
     out = []
     for pipeline in (0, 1):
