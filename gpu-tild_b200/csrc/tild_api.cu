@@ -5,12 +5,64 @@
 // kernels of tild_step.cu and tild_obs.cu.  Errors never exit the process: every call returns
 // a tild_status and records a message on the context.
 #include "tild_internal.cuh"
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
-#include <algorithm>
+#include <mutex>
 
 namespace {
+
+// Page-locked words for the contexts' status copies, 64 bytes each from pages of 64 that are registered once:
+// a page-locked allocation of their own cost every context 1.3 to 3 ms (and some 10 to 300), a third of
+// creating a small one.  The first page stays for the next context, others go when they are empty.  A page
+// that cannot be registered, or no longer is after a device reset, serves as plain memory.
+class StatusWords {
+  struct Page {
+    char* mem;
+    uint64_t used;
+    bool registered;
+  };
+  std::mutex lock;
+  std::vector<Page> pages;
+  static constexpr size_t kWord = 64, kPage = 4096;
+
+ public:
+  int* get() {
+    std::lock_guard<std::mutex> hold(lock);
+    size_t k = 0;
+    while (k < pages.size() && pages[k].used == ~0ull) k++;
+    if (k == pages.size()) {
+      char* mem = static_cast<char*>(aligned_alloc(kPage, kPage));
+      if (!mem) return nullptr;
+      const bool ok = cudaHostRegister(mem, kPage, cudaHostRegisterPortable) == cudaSuccess;
+      if (!ok) cudaGetLastError();
+      pages.push_back({mem, 0, ok});
+    }
+    int bit = 0;
+    while (pages[k].used >> bit & 1) bit++;
+    pages[k].used |= 1ull << bit;
+    return reinterpret_cast<int*>(pages[k].mem + bit * kWord);
+  }
+  void put(int* word) {
+    std::lock_guard<std::mutex> hold(lock);
+    for (size_t k = 0; k < pages.size(); k++) {
+      const ptrdiff_t at = reinterpret_cast<char*>(word) - pages[k].mem;
+      if (at < 0 || at >= (ptrdiff_t)kPage) continue;
+      pages[k].used &= ~(1ull << (at / kWord));
+      if (pages[k].used || k == 0) return;
+      if (pages[k].registered && cudaHostUnregister(pages[k].mem) != cudaSuccess) cudaGetLastError();
+      free(pages[k].mem);
+      pages.erase(pages.begin() + k);
+      return;
+    }
+  }
+};
+StatusWords& status_words() {
+  static StatusWords* words = new StatusWords;  // no CUDA calls at exit
+  return *words;
+}
 
 inline unsigned nblk(long long n, int b) { return (unsigned)((n + b - 1) / b); }
 
@@ -130,7 +182,7 @@ void free_all(tild_ctx* c) {
     }
   for (auto& ge : c->graphs) cudaGraphExecDestroy(ge.exec);
   c->graphs.clear();
-  if (c->h_status) cudaFreeHost(c->h_status);
+  if (c->h_status) status_words().put(c->h_status);
   tild_sort_free(c);
   tild_fft_free(c);
   for (cudaStream_t a : c->aux) cudaStreamDestroy(a);
@@ -596,10 +648,7 @@ int engine_create(const tild_config* cfgs, int nsys, int device, tild_ctx* c, co
   rc = rc ? rc : dalloc(c, &c->kk, (size_t)kd, "k vectors");
   rc = rc ? rc : dalloc(c, &c->xfer, (size_t)maxns * 3, "transfer buffer");
   rc = rc ? rc : dalloc(c, &c->d_status, 2, "status");  // [0] status word, [1] input check flag
-  if (!rc && cudaMallocHost(&c->h_status, 2 * sizeof(int)) != cudaSuccess) {
-    cudaGetLastError();
-    return set_err(c, TILD_ERR_OOM, "page-locked memory for the status word");
-  }
+  if (!rc && !(c->h_status = status_words().get())) return set_err(c, TILD_ERR_OOM, "host memory for the status word");
   rc = rc ? rc : dalloc(c, &c->d_sys, (size_t)nsys, "system descriptors");
   rc = rc ? rc : dalloc(c, &c->cta_bead, tb.size(), "lookup");
   rc = rc ? rc : dalloc(c, &c->cta_spec, tspec.size(), "lookup");

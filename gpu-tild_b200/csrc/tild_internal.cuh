@@ -232,7 +232,7 @@ struct tild_ctx {
   int red_cap = 0;
   float* xfer = nullptr;                 // staging for host transfers, >= 3 * max ns floats
   int* d_status = nullptr;               // [0] status word, [1] input check flag
-  int* h_status = nullptr;               // page-locked copy
+  int* h_status = nullptr;               // page-locked copy (StatusWords)
 
   // spatial sort (tild_sort.cu)
   unsigned* sort_keys = nullptr;
