@@ -347,7 +347,7 @@ def step_bytes(s) -> int:
 # inside the timed region), doubled: the full blend has twice the beads and twice the grid
 # points, and both kernels' traffic grows in proportion.
 NCU_DRAM_BYTES_PER_LAUNCH = {
-    "blend_2.6M_128^3_gaussian_erf_p3_GJF": {"gather": 2 * (119597824 + 15529216), "spread": 2 * (37655040 + 9216)},
+    "blend_2.6M_128^3_gaussian_erf_p3_GJF": {"gather": 2 * (119502592 + 11390720), "spread": 2 * (37652480 + 2304)},
 }
 
 

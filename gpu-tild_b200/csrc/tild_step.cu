@@ -867,8 +867,8 @@ __device__ __forceinline__ void bead_epilogue(int i, const float4& p, int t, flo
 // EARLY (small systems of order <= 1): a launch that leaves SMs with a CTA or two is one chain of
 // latencies, so everything that does not need the field is read and drawn before the stencil (bond
 // partners, x_{n-1}, noise), at the registers of 2 CTAs per SM; and the kernel starts while the grid
-// passes before it end.  us a step: 40^2 film 17.5 -> 16.1, 40^3 with 157 CTAs 30.8 -> 29.8 (30.5 with all
-// reads behind the wait); 235 CTAs of order 4 70.7 -> 72.3 and 860 of order 1 with charges 130 -> 129.
+// passes before it end.  us a step: 40^2 film 17.5 -> 16.1, 40^3 with 157 CTAs 30.8 -> 29.8 (2 us more with
+// all reads behind the wait); 235 CTAs of order 4 70.7 -> 72.3 and 860 of order 1 with charges 130 -> 129.
 //
 // What it reads before its wait (load_done) was last written by an earlier step's gather, a sort, a packing
 // kernel or the counters' kernel.  None of them calls grid_launch_next(), and the gather ends after its own
