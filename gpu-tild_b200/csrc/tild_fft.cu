@@ -628,7 +628,10 @@ __global__ void __launch_bounds__(kThreadsZ, kMinCtasZ) k_fft_z_kmul(const float
   grid_launch_next();  // only now: what starts early from here on (the gather) finds the last step's kernels done
   const SysDev* now = after_wait(&sd);
   const long long est = now->step + ahead + (integrate ? 1 : 0);
-  if (!moves(now, ahead ? ahead : kFirstStep)) return;
+  if (!moves(now, ahead ? ahead : kFirstStep)) {
+    copies_wait();  // the multipliers are still on their way into this block's shared memory
+    return;
+  }
   zk = after_wait(zk);
   if (tile && threadIdx.x < nu) s_scale[threadIdx.x] = sd.zramp[threadIdx.x] < 0 ? 1.f : ramp_ratio(sd, sd.zramp[threadIdx.x], est);
   for (int p0 = 0; p0 < np; p0 += 2) {
